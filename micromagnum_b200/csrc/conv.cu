@@ -68,6 +68,40 @@ mm_status make_twiddles(int n, void **out)
 	return MM_OK;
 }
 
+// Twiddles of a plan's axis: the plain table W_n^k of the mixed-radix passes and, for powers of two,
+// behind it the per-pass tables of the register passes (fft_tw_off) for radix 16 and radix 8.
+constexpr int TW_SETS = 3;
+template <class C>
+__host__ __device__ __forceinline__ const C *tw_of(const C *base, int n, int R)
+{
+	return base + (size_t)n * (R == 8 ? 2 : 1);
+}
+template <typename T>
+mm_status make_pass_twiddles(int n, void **out)
+{
+	std::vector<cplx<T>> h((size_t)n * TW_SETS, cplx<T>{0, 0});
+	for (int k = 0; k < n; ++k) {
+		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
+		h[k].x = (T)cosl(a);
+		h[k].y = (T)sinl(a);
+	}
+	if ((n & (n - 1)) == 0)
+		for (int R : {16, 8}) {
+			if (n < R) continue;
+			cplx<T> *t = h.data() + (tw_of<cplx<T>>(nullptr, n, R) - (const cplx<T> *)nullptr);
+			for (int p = 1, ns = fft_radix(n, R, 0); p < fft_npasses(n, R); ++p) {
+				const int rp = fft_radix(n, R, p);
+				for (int q = 1; q < rp; ++q)
+					for (int jm = 0; jm < ns; ++jm)
+						t[fft_tw_off(n, R, p) + (q - 1) * ns + jm] = h[(size_t)q * jm * (n / (ns * rp))];
+				ns *= rp;
+			}
+		}
+	MM_CUDA(cudaMalloc(out, sizeof(cplx<T>) * h.size()));
+	MM_CUDA(cudaMemcpy(*out, h.data(), sizeof(cplx<T>) * h.size(), cudaMemcpyHostToDevice));
+	return MM_OK;
+}
+
 template <typename T>
 __device__ __forceinline__ void load_twiddles(cplx<T> *tw_s, const cplx<T> *tw_g, int n)
 {
@@ -721,7 +755,7 @@ struct YTmaGeom {
 	static constexpr uint32_t TILE_BYTES = (uint32_t)(TB * ROWS * sizeof(C));
 	static constexpr size_t WORK = ((size_t)SmCols<N, TB, 4>::SIZE * sizeof(C) + 15) / 16 * 16;
 	static constexpr size_t SMEM = 2 * (size_t)TILE_BYTES + WORK + 16;
-	// the single-instance pass keeps the twiddle table W_N^k in shared memory behind the barriers
+	// the single-instance pass keeps its pass twiddles in shared memory behind the barriers
 	static constexpr size_t TW = SMEM;
 	static constexpr size_t SMEM_TW = SMEM + (size_t)N * sizeof(C);
 };
@@ -823,16 +857,17 @@ struct XTmaGeom {
 	static constexpr size_t PER_SM = 228 * 1024;  // shared memory per SM (1 KB of it reserved per CTA)
 	// forward stage: 2 LPB real rows of at most N/2 values and their region bytes
 	static constexpr size_t SB_F = ((size_t)LPB * N * (sizeof(C) / 2 + 1) + 127) / 128 * 128;
-	// forward extras: barriers, the 256-entry Ms table, the twiddle table W_N^k
+	// forward extras: barriers, the 256-entry Ms table, the pass twiddles
 	static constexpr size_t EXTRA_F = 64 + 256 * (sizeof(C) / 2) + (size_t)N * sizeof(C);
 	static constexpr int STG_F = 2 * (3 * SB_F + BUF + EXTRA_F + 1024) <= PER_SM ? 3 : 2;
 	static constexpr size_t SMEM_F = STG_F * SB_F + BUF + EXTRA_F;
 	static constexpr int MINB_F = 2 * (SMEM_F + 1024) <= PER_SM ? 2 : 1;
 	// inverse stage: 2 LPB spectrum rows of lx complex values (lx * sizeof(C) * 2 LPB <= BUF,
-	// checked at set-up); the inverse reads its twiddles from global memory
+	// checked at set-up); behind the work buffer the barriers and the pass twiddles
 	static constexpr size_t SB_I = BUF;
-	static constexpr int STG_I = 2 * (3 * SB_I + BUF + 64 + 1024) <= PER_SM ? 3 : 2;
-	static constexpr size_t SMEM_I = STG_I * SB_I + BUF + 64;
+	static constexpr size_t EXTRA_I = 64 + (size_t)N * sizeof(C);
+	static constexpr int STG_I = 2 * (3 * SB_I + BUF + EXTRA_I + 1024) <= PER_SM ? 3 : 2;
+	static constexpr size_t SMEM_I = STG_I * SB_I + BUF + EXTRA_I;
 	static constexpr int MINB_I = 2 * (SMEM_I + 1024) <= PER_SM ? 2 : 1;
 };
 
@@ -955,6 +990,7 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 	extern __shared__ __align__(128) unsigned char smem_tma[];
 	C *work = reinterpret_cast<C *>(smem_tma + STG * G::SB_I);
 	uint64_t *bar = reinterpret_cast<uint64_t *>(smem_tma + STG * G::SB_I + G::BUF);
+	C *tws = reinterpret_cast<C *>(smem_tma + STG * G::SB_I + G::BUF + 64);
 	const int tid = threadIdx.x;
 	const int line = tid / TPL, j0 = tid % TPL;
 	const int G_ = (int)gridDim.x;
@@ -964,6 +1000,7 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 		mbar_expect_tx(&bar[s], tile_bytes);
 		tma_load_4d(smem_tma + s * G::SB_I, &tmap, 0, 0, row0 % ny, row0 / ny, &bar[s]);
 	};
+	for (int q = tid; q < N; q += blockDim.x) tws[q] = twN[q];
 	if (tid == 0) {
 		for (int s = 0; s < STG; ++s) mbar_init(&bar[s], 1);
 		fence_proxy_async();
@@ -1012,7 +1049,7 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 				issue(next, s);
 			}
 		};
-		cta_fft<T, N, G::R, LPB, true, SI>(work, twN, line, j0, ld, st, release);
+		cta_fft<T, N, G::R, LPB, true, SI>(work, tws, line, j0, ld, st, release);
 	}
 }
 
@@ -1082,7 +1119,7 @@ void fs_y_tma(ConvPlan *p, cudaStream_t st)
 	const int grid = std::min(ntiles, INV ? p->grid_yi : p->grid_yf);
 	k_y_tma<T, N, TB, INV><<<grid, THREADS, G::SMEM_TW, st>>>(INV ? p->tm_yi : p->tm_yf, (C *)p->spec,
 	                                                       INV ? p->ny : N, p->hx, p->lx, tiles_x, ntiles,
-	                                                       (const C *)p->tw_y, p->err);
+	                                                       tw_of((const C *)p->tw_y, N, ct_radix(N)), p->err);
 }
 
 // TMA-staged x passes.  The inverse pass's tensor map (over the spectrum) is fixed; the forward
@@ -1192,11 +1229,11 @@ bool fs_x_fwd_tma(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	if (ms_tab)
 		k_x_fwd_tma<T, N, true><<<grid, G::THREADS, G::SMEM_F, st>>>(*map, *rmap, ms_tab, (C *)p->spec, p->nx, p->ny,
 		                                                            p->nz, p->py, p->hx, p->lx, ntiles,
-		                                                            (const C *)p->tw_x, p->err);
+		                                                            tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err);
 	else
 		k_x_fwd_tma<T, N, false><<<grid, G::THREADS, G::SMEM_F, st>>>(*map, *rmap, ms_tab, (C *)p->spec, p->nx, p->ny,
 		                                                             p->nz, p->py, p->hx, p->lx, ntiles,
-		                                                             (const C *)p->tw_x, p->err);
+		                                                             tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err);
 	return true;
 }
 
@@ -1208,7 +1245,7 @@ void fs_x_inv_tma(ConvPlan *p, T *H, cudaStream_t st)
 	const int ntiles = 3 * p->ny * p->nz / (2 * G::LPB);
 	const int grid = std::min(ntiles, p->grid_xi);
 	k_x_inv_tma<T, N><<<grid, G::THREADS, G::SMEM_I, st>>>(p->tm_xi, H, p->nx, p->ny, p->hx, p->lx, ntiles,
-	                                                     (const C *)p->tw_x, p->err);
+	                                                     tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err);
 }
 
 template <typename T, int N>
@@ -1221,10 +1258,10 @@ void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cuda
 	const size_t smem = (size_t)SmRows<N, LPB>::SIZE * sizeof(C);
 	if (ms_tab)
 		k_x_fwd_ct<T, N, LPB, true><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
-		                                                       p->py, p->hx, p->lx, (const C *)p->tw_x);
+		                                                       p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
 	else
 		k_x_fwd_ct<T, N, LPB, false><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
-		                                                        p->py, p->hx, p->lx, (const C *)p->tw_x);
+		                                                        p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
 }
 
 template <typename T, int N>
@@ -1235,7 +1272,7 @@ void fs_x_inv(ConvPlan *p, T *H, cudaStream_t st)
 	const int lines = (3 * p->ny * p->nz + 1) / 2;
 	const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
 	k_x_inv_ct<T, N, LPB><<<grid, block, (size_t)SmRows<N, LPB>::SIZE * sizeof(C), st>>>(
-	    (const C *)p->spec, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, (const C *)p->tw_x);
+	    (const C *)p->spec, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
 }
 
 template <typename T, int N, bool INV>
@@ -1245,7 +1282,7 @@ void fs_y(ConvPlan *p, cudaStream_t st)
 	constexpr int TB = ct_tb(N, sizeof(C)), TPL = N / ct_radix(N);
 	const dim3 grid((p->hx + TB - 1) / TB, p->nz, 3), block(TB * TPL);
 	k_y_ct<T, N, TB, INV><<<grid, block, (size_t)SmCols<N, TB>::SIZE * sizeof(C), st>>>(
-	    (C *)p->spec, INV ? N : p->ny, INV ? p->ny : N, p->nz, p->hx, p->lx, (const C *)p->tw_y);
+	    (C *)p->spec, INV ? N : p->ny, INV ? p->ny : N, p->nz, p->hx, p->lx, tw_of((const C *)p->tw_y, N, ct_radix(N)));
 }
 
 constexpr int CT_ZTB = 32;
@@ -1256,7 +1293,7 @@ void fs_z(ConvPlan *p, cudaStream_t st)
 	using C = cplx<T>;
 	const dim3 grid((p->hx + CT_ZTB - 1) / CT_ZTB, p->py), block(3 * CT_ZTB * (PZ / ct_radix8(PZ)));
 	k_z_ct<T, PZ, CT_ZTB><<<grid, block, (size_t)SmCols<PZ, 3 * CT_ZTB>::SIZE * sizeof(C), st>>>(
-	    (C *)p->spec, (const T *)p->tensor, p->nz, p->py, p->hx, p->lx, p->qy, p->qz, (const C *)p->tw_z);
+	    (C *)p->spec, (const T *)p->tensor, p->nz, p->py, p->hx, p->lx, p->qy, p->qz, tw_of((const C *)p->tw_z, PZ, ct_radix8(PZ)));
 }
 
 #define MM_FS_SWITCH(n, CALL)                                                                    \
@@ -1380,9 +1417,9 @@ template <typename T>
 mm_status plan_setup(ConvPlan *p, const double *N, cudaStream_t st)
 {
 	using C = cplx<T>;
-	MM_TRY(make_twiddles<T>(p->px, &p->tw_x));
-	MM_TRY(make_twiddles<T>(p->py, &p->tw_y));
-	MM_TRY(make_twiddles<T>(p->pz, &p->tw_z));
+	MM_TRY(make_pass_twiddles<T>(p->px, &p->tw_x));
+	MM_TRY(make_pass_twiddles<T>(p->py, &p->tw_y));
+	MM_TRY(make_pass_twiddles<T>(p->pz, &p->tw_z));
 	MM_CUDA(cudaMalloc(&p->tensor, sizeof(T) * 6 * (size_t)p->qz * p->qy * p->hx));
 	MM_CUDA(cudaMalloc(&p->spec, p->spec_bytes()));
 	MM_CUDA(cudaMemsetAsync(p->spec, 0, p->spec_bytes(), st));
@@ -1724,7 +1761,7 @@ __global__ void __launch_bounds__(LPB * (N / R)) k_x_fwd_grp(const GDesc<T> *__r
 	if (member_skips(d[it.x].flags, gate)) return;
 	const GDesc<T> g = d[it.x];
 	x_fwd_ct_body<T, N, LPB, true, R, true>(g.M[input], g.reg, g.ms_tab, g.spec, g.nx, g.ny, g.nz, g.py, g.hx, g.lx,
-	                                  g.tw_x, it.y);
+	                                  tw_of(g.tw_x, N, R), it.y);
 }
 
 template <typename T, int N, int LPB, int R>
@@ -1735,7 +1772,7 @@ __global__ void __launch_bounds__(LPB * (N / R)) k_x_inv_grp(const GDesc<T> *__r
 	const int2 it = items[blockIdx.x];
 	if (member_skips(d[it.x].flags, gate)) return;
 	const GDesc<T> g = d[it.x];
-	x_inv_ct_body<T, N, LPB, R>(g.spec, g.H[output], g.nx, g.ny, g.nz, g.py, g.hx, g.lx, g.tw_x, it.y);
+	x_inv_ct_body<T, N, LPB, R>(g.spec, g.H[output], g.nx, g.ny, g.nz, g.py, g.hx, g.lx, tw_of(g.tw_x, N, R), it.y);
 }
 
 template <typename T, int N, int TB, bool INV, int R>
@@ -1746,7 +1783,7 @@ __global__ void __launch_bounds__(TB * (N / R)) k_y_grp(const GDesc<T> *__restri
 	if (member_skips(d[it.x].flags, gate)) return;
 	const GDesc<T> g = d[it.x];
 	const int tiles = (g.hx + TB - 1) / TB;
-	y_ct_body<T, N, TB, INV, R>(g.spec, INV ? N : g.ny, INV ? g.ny : N, g.hx, g.lx, g.tw_y, it.y % tiles,
+	y_ct_body<T, N, TB, INV, R>(g.spec, INV ? N : g.ny, INV ? g.ny : N, g.hx, g.lx, tw_of(g.tw_y, N, R), it.y % tiles,
 	                            it.y / tiles);
 }
 
@@ -1845,8 +1882,8 @@ __global__ void __launch_bounds__(ct_tb(N, sizeof(cplx<T>)) * (N / ct_radix(N)),
 				issue(t2, b);
 			}
 		};
-		if constexpr (INV) cta_fft<T, N, R, TB, INV, SI>(work, g.tw_y, line, j0, ld, st, release);
-		else cta_fft_h0<T, N, R, TB, SI>(work, g.tw_y, line, j0, ld, st, release);
+		if constexpr (INV) cta_fft<T, N, R, TB, INV, SI>(work, tw_of(g.tw_y, N, R), line, j0, ld, st, release);
+		else cta_fft_h0<T, N, R, TB, SI>(work, tw_of(g.tw_y, N, R), line, j0, ld, st, release);
 		t = t1;
 		t1 = t2;
 	}
@@ -1985,7 +2022,7 @@ __global__ void __launch_bounds__(YZGeom<PY, PZ, cplx<T>, NARROW>::THREADS)
 		C *sm = smem + (size_t)grp * G::GROUP_ELEMS;
 		auto ld = [&](int ll, int y) -> C { return y < ny ? sm[SI::at(ll, y)] : C{0, 0}; };
 		auto st = [&](int ll, int k, C v) { sm[SI::at(ll, k)] = v; };
-		cta_fft_h0<T, PY, G::R, LG, SI, true>(sm, g.tw_y, line, j0, ld, st);  // rows ny <= PY/2 .. are zero
+		cta_fft_h0<T, PY, G::R, LG, SI, true>(sm, tw_of(g.tw_y, PY, G::R), line, j0, ld, st);  // rows ny <= PY/2 .. are zero
 	}
 	cp_async_wait_group_c<0>();
 	__syncthreads();
@@ -2049,7 +2086,7 @@ __global__ void __launch_bounds__(YZGeom<PY, PZ, cplx<T>, NARROW>::THREADS)
 			if (ok && y < ny) dst[(size_t)y * lx] = val;
 		};
 		if (grp > 0) __syncthreads();
-		cta_fft<T, PY, G::R, LG, true, SI, true>(sm, g.tw_y, line, j0, ld, st);
+		cta_fft<T, PY, G::R, LG, true, SI, true>(sm, tw_of(g.tw_y, PY, G::R), line, j0, ld, st);
 	}
 }
 
