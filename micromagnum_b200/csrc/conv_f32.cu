@@ -1,0 +1,13 @@
+// The convolution's passes in single precision.
+#include "conv_passes.cuh"
+
+namespace mm {
+
+mm_status conv_setup_f32(ConvPlan *p, const double *N, cudaStream_t st) { return plan_setup<float>(p, N, st); }
+
+mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st)
+{
+	return execute<float>(p, M, reg, ms_tab, H, st);
+}
+
+} // namespace mm

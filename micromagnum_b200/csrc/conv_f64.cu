@@ -1,0 +1,13 @@
+// The convolution's passes in double precision.
+#include "conv_passes.cuh"
+
+namespace mm {
+
+mm_status conv_setup_f64(ConvPlan *p, const double *N, cudaStream_t st) { return plan_setup<double>(p, N, st); }
+
+mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st)
+{
+	return execute<double>(p, M, reg, ms_tab, H, st);
+}
+
+} // namespace mm

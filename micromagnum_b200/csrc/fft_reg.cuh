@@ -13,6 +13,9 @@
 #pragma once
 
 #include "fft.cuh"
+#include "mm_common.cuh"
+
+#include <cmath>
 
 namespace mm {
 
@@ -26,8 +29,6 @@ __device__ __forceinline__ double2 w64<double>(int q) { return c_w64d[q]; }
 template <>
 __device__ __forceinline__ float2 w64<float>(int q) { return c_w64f[q]; }
 
-// Uploads the W_64 table to the current device (idempotent).
-mm_status fft_reg_init();
 
 __host__ __device__ constexpr int brev_c(int k, int n)
 {
@@ -220,6 +221,21 @@ __device__ __forceinline__ void cta_fft_h0(cplx<T> *sm, const cplx<T> *__restric
                                            ST &st, HK hk = HK())
 {
 	cta_fft_pass<T, N, R, LANES, false, SmIdx, LD_SM, 0, true>(sm, twp, line, j0, ld, st, hk);
+}
+
+// Uploads this translation unit's tables to the current device (idempotent).
+static inline mm_status fft_reg_init()
+{
+	double2 d[64];
+	float2 f[64];
+	for (int k = 0; k < 64; ++k) {
+		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / 64.0L;
+		d[k] = double2{(double)cosl(a), (double)sinl(a)};
+		f[k] = float2{(float)cosl(a), (float)sinl(a)};
+	}
+	MM_CUDA(cudaMemcpyToSymbol(c_w64d, d, sizeof(d)));
+	MM_CUDA(cudaMemcpyToSymbol(c_w64f, f, sizeof(f)));
+	return MM_OK;
 }
 
 } // namespace mm
