@@ -24,8 +24,10 @@ FftRadices fft_factor(int n)
 // conv_f64.cu, conv_f32.cu
 mm_status conv_setup_f64(ConvPlan *p, const double *N, cudaStream_t st);
 mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st);
+int conv_fit_length_f64(int n, int e, bool z);
 mm_status conv_setup_f32(ConvPlan *p, const double *N, cudaStream_t st);
 mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st);
+int conv_fit_length_f32(int n, int e, bool z);
 
 size_t ConvPlan::spec_bytes() const
 {
@@ -103,15 +105,20 @@ ConvPlan::~ConvPlan()
 
 int conv_launches(const ConvPlan *p) { return p->is2d ? 3 : 5; }
 
-mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int px, int py, int pz,
-                           const double *N, cudaStream_t st)
+mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey, int ez,
+                           const double *N, cudaStream_t st, bool keep_lengths)
 {
 	if (prec != MM_F64 && prec != MM_F32) return fail(MM_ERR_INVALID_ARGUMENT, "conv: bad precision");
-	if (nx <= 0 || ny <= 0 || nz <= 0 || px < nx || py < ny || pz < nz || !N)
+	if (nx <= 0 || ny <= 0 || nz <= 0 || ex < nx || ey < ny || ez < nz || !N)
 		return fail(MM_ERR_INVALID_ARGUMENT, "conv: invalid sizes or null tensor");
+	auto length = [&](int n, int e, bool z) {
+		return keep_lengths ? e : prec == MM_F64 ? conv_fit_length_f64(n, e, z) : conv_fit_length_f32(n, e, z);
+	};
+	const int px = length(nx, ex, false), py = length(ny, ey, false), pz = length(nz, ez, true);
 	ConvPlan *p = new ConvPlan();
 	p->prec = prec;
 	p->nx = nx; p->ny = ny; p->nz = nz;
+	p->ex = ex; p->ey = ey; p->ez = ez;
 	p->px = px; p->py = py; p->pz = pz;
 	p->hx = px / 2 + 1;
 	{

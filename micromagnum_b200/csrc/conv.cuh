@@ -11,13 +11,14 @@ namespace mm {
 struct ConvPlan {
 	int prec = MM_F64;
 	int nx = 0, ny = 0, nz = 0;     // grid
-	int px = 0, py = 0, pz = 0;     // padded (FFT) lengths
+	int ex = 0, ey = 0, ez = 0;     // padded lengths of the tensor's layout
+	int px = 0, py = 0, pz = 0;     // FFT lengths (an axis the tensor pads may take another length)
 	int hx = 0;                     // px/2 + 1 stored x frequencies
 	int lx = 0;                     // spectrum row stride (>= hx complex, rows 16-byte aligned)
 	int xbox_n = 1, xbox_w = 0;     // a spectrum row as xbox_n TMA boxes of xbox_w 8-byte elements
 	int qy = 0, qz = 0;             // py/2 + 1, pz/2 + 1 stored tensor frequencies
 	bool is2d = false;              // nz == 1 && pz == 1
-	bool fast_x = false, fast_y = false, fast_z = false;  // power-of-two register-FFT passes
+	bool fast_x = false, fast_y = false, fast_z = false;  // compile-time register-FFT passes (2^k, 3 * 2^k)
 	bool reg_z = false;             // z pass with whole columns in registers (nz <= pz/2, pz small)
 	bool tma_y = false;             // y passes fed by TMA-staged tiles (persistent CTAs)
 	CUtensorMap tm_yf{}, tm_yi{};   // spectrum views of the forward (ny rows) and inverse (py rows) y pass
@@ -51,9 +52,10 @@ struct ConvPlan {
 };
 
 // Builds the plan and the tensor spectrum from an FP64 tensor in the reference layout
-// (component fastest, then x, y, z) of padded size px*py*pz.
-mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int px, int py,
-                           int pz, const double *N_device, cudaStream_t st);
+// (component fastest, then x, y, z) of padded size ex*ey*ez.  The FFT lengths of zero-padded axes are
+// the plan's choice (keep_lengths: the tensor's own, as the grouped passes need powers of two).
+mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey,
+                           int ez, const double *N_device, cudaStream_t st, bool keep_lengths = false);
 
 // H = N * (Ms[region] * M) when regions/ms_table are given (ms_table: 256 entries), else H = N * M.
 // M and H are SoA arrays of T (T = double for MM_F64, float for MM_F32).

@@ -10,4 +10,6 @@ mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const fl
 	return execute<float>(p, M, reg, ms_tab, H, st);
 }
 
+int conv_fit_length_f32(int n, int e, bool z) { return fit_length<float>(n, e, z); }
+
 } // namespace mm

@@ -10,4 +10,6 @@ mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const d
 	return execute<double>(p, M, reg, ms_tab, H, st);
 }
 
+int conv_fit_length_f64(int n, int e, bool z) { return fit_length<double>(n, e, z); }
+
 } // namespace mm

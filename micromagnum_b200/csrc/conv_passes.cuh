@@ -56,8 +56,9 @@ mm_status make_twiddles(int n, void **out)
 	return MM_OK;
 }
 
-// Twiddles of a plan's axis: the plain table W_n^k of the mixed-radix passes and, for powers of two,
-// behind it the per-pass tables of the register passes (fft_tw_off) for radix 16 and radix 8.
+// Twiddles of a plan's axis: the plain table W_n^k of the mixed-radix passes and, for powers of two
+// (and three times one) behind it the per-pass tables of the register passes (fft_tw_off), the
+// usual radices first, then those of radix 8.
 constexpr int TW_SETS = 3;
 template <class C>
 __host__ __device__ __forceinline__ const C *tw_of(const C *base, int n, int R)
@@ -73,9 +74,9 @@ mm_status make_pass_twiddles(int n, void **out)
 		h[k].x = (T)cosl(a);
 		h[k].y = (T)sinl(a);
 	}
-	if ((n & (n - 1)) == 0)
-		for (int R : {16, 8}) {
-			if (n < R) continue;
+	if (fft_is_pow2(n) || (n % 3 == 0 && fft_is_pow2(n / 3)))
+		for (int R : {fft_is_pow2(n) ? 16 : 24, 8}) {
+			if (n < R || (R == 8 && !fft_is_pow2(n))) continue;
 			cplx<T> *t = h.data() + (tw_of<cplx<T>>(nullptr, n, R) - (const cplx<T> *)nullptr);
 			for (int p = 1, ns = fft_radix(n, R, 0); p < fft_npasses(n, R); ++p) {
 				const int rp = fft_radix(n, R, p);
@@ -373,10 +374,22 @@ __global__ void __launch_bounds__(NT) k_fft_axis(cplx<T> *__restrict__ data, int
 	}
 }
 
-__global__ void k_tensor_component(const double *__restrict__ N, double2 *__restrict__ X, size_t cnt, int comp)
+// One axis of the tensor's layout (length e, negative offsets from the end) at the plan's FFT length
+// p: the source index of entry i, -1 for a zero (offsets beyond n - 1 touch no cell of the box).
+__device__ __forceinline__ int tensor_src(int i, int n, int e, int p)
 {
-	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cnt; i += (size_t)gridDim.x * blockDim.x)
-		X[i] = double2{N[i * 6 + comp], 0.0};
+	if (e == p || i < n) return i;
+	return i > p - n ? e - (p - i) : -1;
+}
+
+__global__ void k_tensor_component(const double *__restrict__ N, double2 *__restrict__ X, int3 n, int3 e, int3 p, int comp)
+{
+	const size_t cnt = (size_t)p.x * p.y * p.z;
+	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < cnt; i += (size_t)gridDim.x * blockDim.x) {
+		const int x = tensor_src((int)(i % p.x), n.x, e.x, p.x), y = tensor_src((int)(i / p.x % p.y), n.y, e.y, p.y),
+		          z = tensor_src((int)(i / ((size_t)p.x * p.y)), n.z, e.z, p.z);
+		X[i] = double2{x < 0 || y < 0 || z < 0 ? 0.0 : N[(((size_t)z * e.y + y) * e.x + x) * 6 + comp], 0.0};
+	}
 }
 
 // Keeps Re of the spectrum on kx < hx, ky <= py/2, kz <= pz/2, scaled by 1/(px py pz), and
@@ -416,7 +429,7 @@ mm_status set_smem(const void *fn, size_t bytes)
 }
 
 // ---- CTA-Stockham passes (cta_fft, radix 16 in registers, shared-memory passes) -----------------
-__host__ __device__ constexpr int ct_radix(int n) { return n < 16 ? n : 16; }
+__host__ __device__ constexpr int ct_radix(int n) { return fft_is_pow2(n) ? (n < 16 ? n : 16) : n < 24 ? n : 24; }
 __host__ __device__ constexpr int ct_radix8(int n) { return n < 8 ? n : 8; }
 __host__ __device__ constexpr int ct_tb(int n, int csize)
 {
@@ -430,6 +443,22 @@ __host__ __device__ constexpr int ct_lpb(int n, int csize)
 	if (l < 1) l = 1;
 	while (l > 1 && (long)(l * n + (l * n >> 5) + 1) * csize > 65536) l >>= 1;
 	return l;
+}
+
+// Tiles of a grid that would not fill the device with the sizes above: one warp's worth of lines,
+// and rows of at least 32 bytes in the y pass.  A 128x32 film has 48 lines in its x passes, 3 CTAs of
+// 16 lines, each waiting on its own passes: 24 CTAs of 2 lines take 12.8 us forward, FP64, against
+// 14.0 (event-timed, about 6 us of it the timing).
+__host__ __device__ constexpr int ct_lpb_narrow(int n)
+{
+	const int l = 32 / (n / ct_radix(n));
+	return l < 1 ? 1 : l;
+}
+__host__ __device__ constexpr int ct_tb_narrow(int n, int csize)
+{
+	int tb = 32 / csize;
+	while (tb * (n / ct_radix(n)) < 32) tb <<= 1;
+	return tb < ct_tb(n, csize) ? tb : ct_tb(n, csize);
 }
 
 // y pass (3-D): TB columns per CTA; forward pads rows n_in -> N, inverse crops N -> n_out.
@@ -496,7 +525,7 @@ __device__ __forceinline__ void x_fwd_ct_body(const T *__restrict__ M, const uin
 	C *Sb = S + ((size_t)(qb / nyz * nz + qb % nyz / ny) * py + qb % nyz % ny) * lx;
 	const T h = T(0.5);
 	for (int k = j0; k < hx; k += TPL) {
-		const C zk = sm[SI::at(line, k)], zn = sm[SI::at(line, (N - k) & (N - 1))];
+		const C zk = sm[SI::at(line, k)], zn = sm[SI::at(line, k == 0 ? 0 : N - k)];
 		if (va) Sa[k] = C{h * (zk.x + zn.x), h * (zk.y - zn.y)};
 		if (vb) Sb[k] = C{h * (zk.y + zn.y), h * (zn.x - zk.x)};
 	}
@@ -555,6 +584,64 @@ __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_inv_ct(const cplx
                                                                      const cplx<T> *__restrict__ twN)
 {
 	x_inv_ct_body<T, N, LPB>(S, H, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
+}
+
+// y pass with the tensor multiply for 2-D problems (CTA-Stockham form): a CTA takes TB columns of
+// x-frequencies of all three components (lines c * TB + b), transforms them along y into shared
+// memory, and the inverse transform's first pass reads its inputs through the tensor (three
+// components and three tensor entries per value), so the y spectrum never leaves the SM.  Bound by
+// the latency of its passes for films of up to a few ten thousand cells: 128x32 cells, FP64, 8.6 us
+// against 18.7 in the mixed-radix form (5 CTAs of 32 columns), 500x125 cells 14.7 against 27.2
+// (event-timed, about 6 us of it the timing).
+__host__ __device__ constexpr int y2d_tb(int n, int csize)
+{
+	int tb = 8;
+	while (tb > 1 && (3L * tb * n * csize > 100 * 1024 || 3 * tb * (n / ct_radix(n)) > (csize == 8 ? 768 : 512))) tb >>= 1;
+	return tb;
+}
+
+template <typename T, int N, int TB>
+__global__ void __launch_bounds__(3 * TB * (N / ct_radix(N)))
+    k_y2d_ct(cplx<T> *__restrict__ S, const T *__restrict__ Nt, int ny, int hx, int lx, int qy,
+             const cplx<T> *__restrict__ twN)
+{
+	using C = cplx<T>;
+	constexpr int R = ct_radix(N), LANES = 3 * TB;
+	using SI = SmCols<N, LANES>;
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	C *sm = reinterpret_cast<C *>(smem_raw);
+	const int tid = threadIdx.x;
+	const int line = tid % LANES, j0 = tid / LANES;
+	const int c = line / TB, b = line % TB;
+	const int kx = blockIdx.x * TB + b;
+	const bool ok = kx < hx;
+	C *col = S + (size_t)c * N * lx + (ok ? kx : 0);
+	{
+		auto ld = [&](int, int y) -> C { return (ok && y < ny) ? col[(size_t)y * lx] : C{0, 0}; };
+		auto st = [&](int l, int k, C v) { sm[SI::at(l, k)] = v; };
+		cta_fft<T, N, R, LANES, false, SI>(sm, twN, line, j0, ld, st);
+	}
+	__syncthreads();
+	// row c of the symmetric tensor (components xx, xy, xz, yy, yz, zz); xy and yz are odd in ky
+	const size_t cs = (size_t)qy * hx;
+	const T *t0 = Nt + (size_t)c * cs + (ok ? kx : 0);
+	const T *t1 = Nt + (size_t)(c == 0 ? 1 : c + 2) * cs + (ok ? kx : 0);
+	const T *t2 = Nt + (size_t)(c == 0 ? 2 : c + 3) * cs + (ok ? kx : 0);
+	auto ld = [&](int, int k) -> C {
+		const bool f = 2 * k > N;
+		const size_t r = (size_t)(f ? N - k : k) * hx;
+		const T s = f ? T(-1) : T(1);
+		T n0 = t0[r], n1 = t1[r], n2 = t2[r];
+		if (c == 0) n1 = s * n1;
+		else if (c == 1) { n0 = s * n0; n2 = s * n2; }
+		else n1 = s * n1;
+		const C m0 = sm[SI::at(b, k)], m1 = sm[SI::at(TB + b, k)], m2 = sm[SI::at(2 * TB + b, k)];
+		return C{n0 * m0.x + n1 * m1.x + n2 * m2.x, n0 * m0.y + n1 * m1.y + n2 * m2.y};
+	};
+	auto st = [&](int, int y, C v) {
+		if (ok && y < ny) col[(size_t)y * lx] = v;
+	};
+	cta_fft<T, N, R, LANES, true, SI, true>(sm, twN, line, j0, ld, st);
 }
 
 // z pass with the tensor multiply (CTA-Stockham form): lines (c, b) = c * TB + b hold the z
@@ -675,7 +762,7 @@ __device__ __forceinline__ void z_reg_body(cplx<T> *__restrict__ S, const T *__r
 	dft_reg_halfzero<T, PZ>(v);
 	C *mine = sm + (r * PZ * 3 + c) * 32 + lane;
 #pragma unroll
-	for (int k = 0; k < PZ; ++k) mine[brev<PZ>(k) * 96] = v[k];
+	for (int k = 0; k < PZ; ++k) mine[k * 96] = v[dft_pos<PZ>(k)];
 	cp_async_wait_all_t();
 	__syncthreads();
 	if (kx < hx) {
@@ -708,7 +795,7 @@ __device__ __forceinline__ void z_reg_body(cplx<T> *__restrict__ S, const T *__r
 	if (ok) {
 #pragma unroll
 		for (int z = 0; z < H; ++z)
-			if (z < nz) col[z * zstride] = v[brev<PZ>(z)];
+			if (z < nz) col[z * zstride] = v[dft_pos<PZ>(z)];
 	}
 }
 
@@ -737,7 +824,8 @@ void fs_z_reg(ConvPlan *p, cudaStream_t st)
 template <int N, int TB, bool INV, class C>
 struct YTmaGeom {
 	static constexpr int ROWS = INV ? N : N / 2;
-	static constexpr int BR = ROWS < 256 ? ROWS : 256;
+	static constexpr int BR = ROWS < 256 ? ROWS : ROWS % 256 == 0 ? 256 : 192;  // rows of a box
+	static_assert(ROWS % BR == 0, "a tile is whole boxes");
 	static constexpr int NBOX = ROWS / BR;
 	static constexpr int E = (int)(sizeof(C) / 8);
 	static constexpr uint32_t TILE_BYTES = (uint32_t)(TB * ROWS * sizeof(C));
@@ -753,7 +841,8 @@ struct YTmaGeom {
 __host__ __device__ constexpr int y_tma_tb(int n, int csize)
 {
 	int tb = ct_tb(n, csize);
-	while (tb * csize > 32 && tb * (n / ct_radix(n)) > 256) tb >>= 1;
+	while (tb * csize > 32 && (tb * (n / ct_radix(n)) > 256 || (!fft_is_pow2(n) && 3L * n * tb * csize > 110 * 1024)))
+		tb >>= 1;
 	return tb;
 }
 
@@ -957,7 +1046,7 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 		C *Sb = S + ((size_t)(qb / nyz * nz + qb % nyz / ny) * py + qb % nyz % ny) * lx;
 		const T h = T(0.5);
 		for (int kk = j0; kk < hx; kk += TPL) {
-			const C zk = work[SI::at(line, kk)], zn = work[SI::at(line, (N - kk) & (N - 1))];
+			const C zk = work[SI::at(line, kk)], zn = work[SI::at(line, kk == 0 ? 0 : N - kk)];
 			if (va) Sa[kk] = C{h * (zk.x + zn.x), h * (zk.y - zn.y)};
 			if (vb) Sb[kk] = C{h * (zk.y + zn.y), h * (zn.x - zk.x)};
 		}
@@ -1044,25 +1133,78 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 // ---- fast-path geometry and dispatch ---------------------------------------------------------------
 
 
+// Lengths with compile-time passes: powers of two and three times powers of two.
 template <typename T>
 bool fs_len_ok(int n)
 {
-	if (n < 4 || (n & (n - 1))) return false;
-	return sizeof(T) == 4 ? n <= 2048 : n <= 1024;
+	if (fft_is_pow2(n)) return n >= 4 && n <= 2048;
+	return n % 3 == 0 && fft_is_pow2(n / 3) && n >= 12 && n <= 1536;
+}
+
+// z lengths with compile-time passes: whole columns in registers (zero-padded axes), or through
+// shared memory (powers of two, padded or not).
+template <typename T>
+bool fz_reg_ok(int pz, int nz)
+{
+	if (2 * nz > pz) return false;
+	if (fft_is_pow2(pz)) return pz >= 2 && pz <= (sizeof(T) == 4 ? 32 : 16);
+	return pz == 6 || pz == 12 || pz == 24;
+}
+template <typename T>
+bool fz_len_ok(int pz, int nz)
+{
+	return fz_reg_ok<T>(pz, nz) || (fft_is_pow2(pz) && pz >= 2 && pz <= 64);
+}
+
+// FFT length of one axis of n cells whose tensor layout has length e.  With e >= 2n - 1 the axis is
+// zero padded and any length >= 2n - 1 gives the same convolution, so it takes the shortest length
+// with compile-time passes (2n or more, whose upper half of inputs is zero) instead of the
+// mixed-radix passes at e; otherwise the convolution is circular and e is its length.  The
+// run-time radices of the mixed-radix passes cost an integer division per index and one barrier
+// per small radix: 200x150x6 cells, FP32, took 27 + 52 + 29 us in the y, z and y passes at 300 and 12
+// points and 24 + 27 us in the x passes at 400; at 384, 12 and 512 points the compile-time passes
+// take 15 + 13 + 15 and 15 + 11 us (event-timed, about 6 us of each is the timing).  A length with a large
+// prime factor gained most (796 points: 980 us a pass, against 15 at 1024).
+template <typename T>
+int fit_length(int n, int e, bool z)
+{
+	if (n < 2 || e < 2 * n - 1) return e;
+	int best = 0;
+	for (int base : {1, 3})
+		for (int len = base == 3 ? 6 : 2; len <= 2048; len *= 2)
+			if (len >= 2 * n && (z ? fz_len_ok<T>(len, n) : fs_len_ok<T>(len)) && (best == 0 || len < best)) best = len;
+	return best ? best : e;
 }
 
 template <typename T, int N>
 mm_status fs_setup_len()
 {
 	using C = cplx<T>;
-	constexpr int TB = ct_tb(N, sizeof(C)), LPB = ct_lpb(N, sizeof(C));
+	constexpr int TB = ct_tb(N, sizeof(C)), LPB = ct_lpb(N, sizeof(C)), T2 = y2d_tb(N, sizeof(C));
 	const size_t sx = (size_t)SmRows<N, LPB>::SIZE * sizeof(C), sy = (size_t)SmCols<N, TB>::SIZE * sizeof(C);
+	MM_TRY(set_smem<T>((const void *)k_y2d_ct<T, N, T2>, (size_t)SmCols<N, 3 * T2>::SIZE * sizeof(C)));
+	MM_TRY(set_smem<T>((const void *)k_y2d_ct<T, N, 1>, (size_t)SmCols<N, 3>::SIZE * sizeof(C)));
 	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, false>, sx));
 	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, true>, sx));
 	MM_TRY(set_smem<T>((const void *)k_x_inv_ct<T, N, LPB>, sx));
 	MM_TRY(set_smem<T>((const void *)k_y_ct<T, N, TB, false>, sy));
 	MM_TRY(set_smem<T>((const void *)k_y_ct<T, N, TB, true>, sy));
 	return MM_OK;
+}
+
+// Whether the usual tiles of the x or y passes leave SMs without work: then narrow tiles spread the
+// lines over the device (and the staged passes, whose CTAs walk several tiles each, are not used).
+template <typename T, int N>
+bool fs_narrow_x(const ConvPlan *p)
+{
+	constexpr int LPB = ct_lpb(N, sizeof(cplx<T>));
+	return ((3 * p->ny * p->nz + 1) / 2 + LPB - 1) / LPB < num_sms();
+}
+template <typename T, int N>
+bool fs_narrow_y(const ConvPlan *p)
+{
+	constexpr int TB = ct_tb(N, sizeof(cplx<T>));
+	return (p->hx + TB - 1) / TB * 3 * p->nz < num_sms();
 }
 
 // TMA-staged y passes: tensor maps over the spectrum, shared-memory size, persistent grid size.
@@ -1076,6 +1218,7 @@ mm_status fs_setup_y_tma(ConvPlan *p)
 	using GF = YTmaGeom<N, TB, false, C>;
 	using GI = YTmaGeom<N, TB, true, C>;
 	p->tma_y = false;
+	if (fs_narrow_y<T, N>(p)) return MM_OK;
 	if (GI::SMEM_TW > 227 * 1024 || 2 * p->ny > p->py || TB * sizeof(C) < 16) return MM_OK;
 	constexpr int E = GF::E;
 	const uint64_t d0 = (uint64_t)p->lx * E, rowb = (uint64_t)p->lx * sizeof(C), planeb = rowb * p->py;
@@ -1120,6 +1263,7 @@ mm_status fs_setup_x_tma(ConvPlan *p)
 	using G = XTmaGeom<N, C>;
 	constexpr int LPB = G::LPB;
 	p->tma_xf = p->tma_xi = false;
+	if (fs_narrow_x<T, N>(p)) return MM_OK;
 	// the forward pass's half-zero first butterflies need nx <= N/2 (non-periodic zero padding)
 	if (G::SMEM_F > 227 * 1024 || G::SMEM_I > 227 * 1024 || N < 64 || 2 * p->nx > N) return MM_OK;
 	int occ = 0;
@@ -1240,37 +1384,69 @@ template <typename T, int N>
 void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cudaStream_t st)
 {
 	using C = cplx<T>;
-	constexpr int LPB = ct_lpb(N, sizeof(C)), TPL = N / ct_radix(N);
+	constexpr int TPL = N / ct_radix(N);
 	const int lines = (3 * p->ny * p->nz + 1) / 2;
-	const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
-	const size_t smem = (size_t)SmRows<N, LPB>::SIZE * sizeof(C);
-	if (ms_tab)
-		k_x_fwd_ct<T, N, LPB, true><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
+	auto go = [&](auto lpb) {
+		constexpr int LPB = decltype(lpb)::value;
+		const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
+		const size_t smem = (size_t)SmRows<N, LPB>::SIZE * sizeof(C);
+		if (ms_tab)
+			k_x_fwd_ct<T, N, LPB, true><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
 		                                                       p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
-	else
-		k_x_fwd_ct<T, N, LPB, false><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
-		                                                        p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+		else
+			k_x_fwd_ct<T, N, LPB, false><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
+			                                                        p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+	};
+	if (fs_narrow_x<T, N>(p)) go(std::integral_constant<int, ct_lpb_narrow(N)>());
+	else go(std::integral_constant<int, ct_lpb(N, sizeof(C))>());
 }
 
 template <typename T, int N>
 void fs_x_inv(ConvPlan *p, T *H, cudaStream_t st)
 {
 	using C = cplx<T>;
-	constexpr int LPB = ct_lpb(N, sizeof(C)), TPL = N / ct_radix(N);
+	constexpr int TPL = N / ct_radix(N);
 	const int lines = (3 * p->ny * p->nz + 1) / 2;
-	const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
-	k_x_inv_ct<T, N, LPB><<<grid, block, (size_t)SmRows<N, LPB>::SIZE * sizeof(C), st>>>(
-	    (const C *)p->spec, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+	auto go = [&](auto lpb) {
+		constexpr int LPB = decltype(lpb)::value;
+		const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
+		k_x_inv_ct<T, N, LPB><<<grid, block, (size_t)SmRows<N, LPB>::SIZE * sizeof(C), st>>>(
+		    (const C *)p->spec, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+	};
+	if (fs_narrow_x<T, N>(p)) go(std::integral_constant<int, ct_lpb_narrow(N)>());
+	else go(std::integral_constant<int, ct_lpb(N, sizeof(C))>());
 }
 
 template <typename T, int N, bool INV>
 void fs_y(ConvPlan *p, cudaStream_t st)
 {
 	using C = cplx<T>;
-	constexpr int TB = ct_tb(N, sizeof(C)), TPL = N / ct_radix(N);
-	const dim3 grid((p->hx + TB - 1) / TB, p->nz, 3), block(TB * TPL);
-	k_y_ct<T, N, TB, INV><<<grid, block, (size_t)SmCols<N, TB>::SIZE * sizeof(C), st>>>(
-	    (C *)p->spec, INV ? N : p->ny, INV ? p->ny : N, p->nz, p->hx, p->lx, tw_of((const C *)p->tw_y, N, ct_radix(N)));
+	constexpr int TPL = N / ct_radix(N);
+	auto go = [&](auto tb) {
+		constexpr int TB = decltype(tb)::value;
+		const dim3 grid((p->hx + TB - 1) / TB, p->nz, 3), block(TB * TPL);
+		k_y_ct<T, N, TB, INV><<<grid, block, (size_t)SmCols<N, TB>::SIZE * sizeof(C), st>>>(
+		    (C *)p->spec, INV ? N : p->ny, INV ? p->ny : N, p->nz, p->hx, p->lx,
+		    tw_of((const C *)p->tw_y, N, ct_radix(N)));
+	};
+	if (fs_narrow_y<T, N>(p)) go(std::integral_constant<int, ct_tb_narrow(N, sizeof(C))>());
+	else go(std::integral_constant<int, ct_tb(N, sizeof(C))>());
+}
+
+// The fused y pass of a 2-D problem: tiles of several columns where they fill the device, else single
+// columns.
+template <typename T, int N>
+void fs_y2d(ConvPlan *p, cudaStream_t st)
+{
+	using C = cplx<T>;
+	constexpr int TPL = N / ct_radix(N), WIDE = y2d_tb(N, sizeof(C));
+	auto go = [&](auto tb) {
+		constexpr int TB = decltype(tb)::value;
+		k_y2d_ct<T, N, TB><<<(p->hx + TB - 1) / TB, 3 * TB * TPL, (size_t)SmCols<N, 3 * TB>::SIZE * sizeof(C), st>>>(
+		    (C *)p->spec, (const T *)p->tensor, p->ny, p->hx, p->lx, p->qy, tw_of((const C *)p->tw_y, N, ct_radix(N)));
+	};
+	if (p->hx >= WIDE * num_sms()) go(std::integral_constant<int, WIDE>());
+	else go(std::integral_constant<int, 1>());
 }
 
 constexpr int CT_ZTB = 32;
@@ -1299,31 +1475,49 @@ void fs_z(ConvPlan *p, cudaStream_t st)
 	default: break;                                                                              \
 	}
 
+// The lengths of fs_len_ok: the single-instance passes (grouped members have power-of-two lengths).
+#define MM_FS_SWITCH3(n, CALL)                                                                   \
+	switch (n) {                                                                                 \
+	case 12: CALL(12); break;                                                                    \
+	case 24: CALL(24); break;                                                                    \
+	case 48: CALL(48); break;                                                                    \
+	case 96: CALL(96); break;                                                                    \
+	case 192: CALL(192); break;                                                                  \
+	case 384: CALL(384); break;                                                                  \
+	case 768: CALL(768); break;                                                                  \
+	case 1536: CALL(1536); break;                                                                \
+	case 2048: CALL(2048); break;                                                                \
+	default: MM_FS_SWITCH(n, CALL)                                                               \
+	}
+
 template <typename T>
 mm_status fs_setup(ConvPlan *p)
 {
 	MM_TRY(fft_reg_init());
-	// the power-of-two passes skip the zero upper half of a forward transform, so an axis without
-	// zero padding (a periodic one, padded length n) takes the generic mixed-radix passes
-	p->fast_x = fs_len_ok<T>(p->px) && 2 * p->nx <= p->px;
-	p->fast_y = !p->is2d && fs_len_ok<T>(p->py) && 2 * p->ny <= p->py;
-	p->fast_z = !p->is2d && p->pz >= 2 && p->pz <= 64 && (p->pz & (p->pz - 1)) == 0 && 2 * p->nz <= p->pz;
+	// (the staged and register passes skip the zero upper half of a forward transform; an axis without
+	// zero padding, a periodic one of padded length n, takes those that load every input)
+	p->fast_x = fs_len_ok<T>(p->px);
+	p->fast_y = fs_len_ok<T>(p->py);
+	p->fast_z = !p->is2d && fz_len_ok<T>(p->pz, p->nz);
 	mm_status r = MM_OK;
 #define MM_SETUP(N) r = fs_setup_len<T, N>()
-	if (p->fast_x) { MM_FS_SWITCH(p->px, MM_SETUP); MM_TRY(r); }
-	if (p->fast_y) { MM_FS_SWITCH(p->py, MM_SETUP); MM_TRY(r); }
+	if (p->fast_x) { MM_FS_SWITCH3(p->px, MM_SETUP); MM_TRY(r); }
+	if (p->fast_y) { MM_FS_SWITCH3(p->py, MM_SETUP); MM_TRY(r); }
 #undef MM_SETUP
 #define MM_XTSETUP(N) r = fs_setup_x_tma<T, N>(p)
-	if (p->fast_x) { MM_FS_SWITCH(p->px, MM_XTSETUP); MM_TRY(r); }
+	if (p->fast_x) { MM_FS_SWITCH3(p->px, MM_XTSETUP); MM_TRY(r); }
 #undef MM_XTSETUP
 #define MM_YTSETUP(N) r = fs_setup_y_tma<T, N>(p)
-	if (p->fast_y) { MM_FS_SWITCH(p->py, MM_YTSETUP); MM_TRY(r); }
+	if (p->fast_y && !p->is2d) { MM_FS_SWITCH3(p->py, MM_YTSETUP); MM_TRY(r); }
 #undef MM_YTSETUP
-	p->reg_z = p->fast_z && 2 * p->nz <= p->pz && p->pz <= (sizeof(T) == 4 ? 32 : 16);
+	p->reg_z = p->fast_z && fz_reg_ok<T>(p->pz, p->nz);
 	if (p->reg_z) {
 		const size_t sz = zr_smem<T>(p->pz);
 		switch (p->pz) {
 		case 2: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 2>, sz)); break;
+		case 6: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 6>, sz)); break;
+		case 12: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 12>, sz)); break;
+		case 24: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 24>, sz)); break;
 		case 4: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 4>, sz)); break;
 		case 8: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 8>, sz)); break;
 		case 16: MM_TRY(set_smem<T>((const void *)k_z_reg<T, 16>, sz)); break;
@@ -1361,7 +1555,8 @@ mm_status tensor_spectrum(ConvPlan *p, const double *N, cudaStream_t st)
 	const size_t per = (size_t)p->qz * p->qy * p->hx;
 	const int gsz = num_sms() * 8;
 	for (int comp = 0; comp < 6 && st_ == MM_OK; ++comp) {
-		k_tensor_component<<<gsz, NT, 0, st>>>(N, X, cnt, comp);
+		k_tensor_component<<<gsz, NT, 0, st>>>(N, X, make_int3(p->nx, p->ny, p->nz), make_int3(p->ex, p->ey, p->ez),
+		                                       make_int3(px, py, pz), comp);
 		st_ = after_launch("k_tensor_component");
 		const int dims[3] = {px, py, pz};
 		const FftRadices rads[3] = {p->rx, p->ry, p->rz};
@@ -1427,19 +1622,23 @@ mm_status plan_setup(ConvPlan *p, const double *N, cudaStream_t st)
 		p->tb_z = pick_tile(p->pz, 3, sizeof(C), 32);
 		p->smem_z = (size_t)(6 * p->tb_z + 1) * p->pz * sizeof(C);
 	}
-	if (p->smem_x > 227 * 1024 || p->smem_y > 227 * 1024 || p->smem_z > 227 * 1024)
+	MM_TRY(fs_setup<T>(p));
+	// the mixed-radix passes of the axes without compile-time ones
+	if ((!p->fast_x && p->smem_x > 227 * 1024) || (!p->fast_y && p->smem_y > 227 * 1024) ||
+	    (!p->is2d && !p->fast_z && p->smem_z > 227 * 1024))
 		return fail(MM_ERR_UNSUPPORTED, "conv: FFT length too large for one CTA");
-	MM_TRY(set_smem<T>((const void *)k_x_fwd<T, false>, p->smem_x));
-	MM_TRY(set_smem<T>((const void *)k_x_fwd<T, true>, p->smem_x));
-	MM_TRY(set_smem<T>((const void *)k_x_inv<T>, p->smem_x));
-	if (p->is2d) {
+	if (!p->fast_x) {
+		MM_TRY(set_smem<T>((const void *)k_x_fwd<T, false>, p->smem_x));
+		MM_TRY(set_smem<T>((const void *)k_x_fwd<T, true>, p->smem_x));
+		MM_TRY(set_smem<T>((const void *)k_x_inv<T>, p->smem_x));
+	}
+	if (!p->fast_y && p->is2d) {
 		MM_TRY(set_smem<T>((const void *)k_y_mul2d<T>, p->smem_y));
-	} else {
+	} else if (!p->fast_y) {
 		MM_TRY(set_smem<T>((const void *)k_y<T, false>, p->smem_y));
 		MM_TRY(set_smem<T>((const void *)k_y<T, true>, p->smem_y));
-		MM_TRY(set_smem<T>((const void *)k_z_mul<T>, p->smem_z));
 	}
-	MM_TRY(fs_setup<T>(p));
+	if (!p->is2d && !p->fast_z) MM_TRY(set_smem<T>((const void *)k_z_mul<T>, p->smem_z));
 	return tensor_spectrum<T>(p, N, st);
 }
 
@@ -1460,13 +1659,13 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	bool staged = false;
 	if (p->tma_xf) {
 #define MM_XTF(N) staged = fs_x_fwd_tma<T, N>(p, M, reg, ms_tab, st)
-		MM_FS_SWITCH(p->px, MM_XTF);
+		MM_FS_SWITCH3(p->px, MM_XTF);
 #undef MM_XTF
 	}
 	if (staged) {
 	} else if (p->fast_x) {
 #define MM_XF(N) fs_x_fwd<T, N>(p, M, reg, ms_tab, st)
-		MM_FS_SWITCH(p->px, MM_XF);
+		MM_FS_SWITCH3(p->px, MM_XF);
 #undef MM_XF
 	} else if (ms_tab)
 		k_x_fwd<T, true><<<gx, NT, p->smem_x, st>>>(M, reg, ms_tab, S, p->nx, p->ny, p->nz, p->py, p->hx, p->lx,
@@ -1480,20 +1679,26 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	if (p->is2d) {
 		const int gy = (p->hx + p->tb_y - 1) / p->tb_y;
 		tk = prof_begin(st);
-		k_y_mul2d<T><<<gy, NT, p->smem_y, st>>>(S, (const T *)p->tensor, p->ny, p->hx, p->lx, p->qy, p->ry,
-		                                        (const C *)p->tw_y, p->tb_y);
-		MM_TRY(after_launch("k_y_mul2d"));
-		prof_end(tk, "k_y_mul2d", 2 * half + tens, st);
+		if (p->fast_y) {
+#define MM_Y2(N) fs_y2d<T, N>(p, st)
+			MM_FS_SWITCH3(p->py, MM_Y2);
+#undef MM_Y2
+		} else
+			k_y_mul2d<T><<<gy, NT, p->smem_y, st>>>(S, (const T *)p->tensor, p->ny, p->hx, p->lx, p->qy, p->ry,
+			                                        (const C *)p->tw_y, p->tb_y);
+		const char *y2_name = p->fast_y ? "k_y2d_ct" : "k_y_mul2d";
+		MM_TRY(after_launch(y2_name));
+		prof_end(tk, y2_name, 2 * half + tens, st);
 	} else {
 		dim3 gy((p->hx + p->tb_y - 1) / p->tb_y, p->nz, 3);
 		tk = prof_begin(st);
 		if (p->tma_y) {
 #define MM_YTF(N) fs_y_tma<T, N, false>(p, st)
-			MM_FS_SWITCH(p->py, MM_YTF);
+			MM_FS_SWITCH3(p->py, MM_YTF);
 #undef MM_YTF
 		} else if (p->fast_y) {
 #define MM_YF(N) fs_y<T, N, false>(p, st)
-			MM_FS_SWITCH(p->py, MM_YF);
+			MM_FS_SWITCH3(p->py, MM_YF);
 #undef MM_YF
 		} else
 			k_y<T, false><<<gy, NT, p->smem_y, st>>>(S, p->ny, p->py, p->nz, p->py, p->hx, p->lx, p->ry,
@@ -1506,6 +1711,9 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 		if (p->reg_z) {
 			switch (p->pz) {
 			case 2: fs_z_reg<T, 2>(p, st); break;
+			case 6: fs_z_reg<T, 6>(p, st); break;
+			case 12: fs_z_reg<T, 12>(p, st); break;
+			case 24: fs_z_reg<T, 24>(p, st); break;
 			case 4: fs_z_reg<T, 4>(p, st); break;
 			case 8: fs_z_reg<T, 8>(p, st); break;
 			case 16: fs_z_reg<T, 16>(p, st); break;
@@ -1529,11 +1737,11 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 		tk = prof_begin(st);
 		if (p->tma_y) {
 #define MM_YTI(N) fs_y_tma<T, N, true>(p, st)
-			MM_FS_SWITCH(p->py, MM_YTI);
+			MM_FS_SWITCH3(p->py, MM_YTI);
 #undef MM_YTI
 		} else if (p->fast_y) {
 #define MM_YI(N) fs_y<T, N, true>(p, st)
-			MM_FS_SWITCH(p->py, MM_YI);
+			MM_FS_SWITCH3(p->py, MM_YI);
 #undef MM_YI
 		} else
 			k_y<T, true><<<gy, NT, p->smem_y, st>>>(S, p->py, p->ny, p->nz, p->py, p->hx, p->lx, p->ry,
@@ -1545,11 +1753,11 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	tk = prof_begin(st);
 	if (p->tma_xi) {
 #define MM_XTI(N) fs_x_inv_tma<T, N>(p, H, st)
-		MM_FS_SWITCH(p->px, MM_XTI);
+		MM_FS_SWITCH3(p->px, MM_XTI);
 #undef MM_XTI
 	} else if (p->fast_x) {
 #define MM_XI(N) fs_x_inv<T, N>(p, H, st)
-		MM_FS_SWITCH(p->px, MM_XI);
+		MM_FS_SWITCH3(p->px, MM_XI);
 #undef MM_XI
 	} else
 		k_x_inv<T><<<gx, NT, p->smem_x, st>>>(S, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, p->rx,

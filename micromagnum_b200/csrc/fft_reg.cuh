@@ -1,8 +1,8 @@
 // Register-resident FFT building blocks for power-of-two lengths (included by conv.cu only).
 //
 // dft_reg<T, N, INV>: an N-point DFT (N = 1..64) held entirely in one thread's registers,
-// radix-2 decimation in frequency, fully unrolled, output in bit-reversed order (read it with
-// brev<N>(k)).  Its twiddles W_64^q = exp(-2 pi i q / 64) live in a __constant__ table that every
+// radix-2 decimation in frequency (after one radix-3 stage for N = 3 * 2^k <= 48), fully unrolled,
+// output k in register dft_pos<N>(k).  Its twiddles W_64^q = exp(-2 pi i q / 64) live in a __constant__ table that every
 // lane reads at the same compile-time index (a broadcast).
 //
 // Longer transforms (N = N1 * N2 <= 4096) use the four-step decomposition within a CTA:
@@ -29,6 +29,19 @@ __device__ __forceinline__ double2 w64<double>(int q) { return c_w64d[q]; }
 template <>
 __device__ __forceinline__ float2 w64<float>(int q) { return c_w64f[q]; }
 
+// W_48^q for the register transforms of 3 * 2^k points.
+static __constant__ double2 c_w48d[48];
+static __constant__ float2 c_w48f[48];
+
+template <typename T>
+__device__ __forceinline__ cplx<T> w48(int q);
+template <>
+__device__ __forceinline__ double2 w48<double>(int q) { return c_w48d[q]; }
+template <>
+__device__ __forceinline__ float2 w48<float>(int q) { return c_w48f[q]; }
+
+
+__host__ __device__ constexpr bool fft_is_pow2(int n) { return (n & (n - 1)) == 0; }
 
 __host__ __device__ constexpr int brev_c(int k, int n)
 {
@@ -39,6 +52,15 @@ __host__ __device__ constexpr int brev_c(int k, int n)
 
 template <int N>
 __device__ __forceinline__ int brev(int k) { return brev_c(k, N); }
+
+// Register that holds output k of an N-point register transform: bit-reversed for a power of two;
+// for N = 3 M the outputs 3 k' + r are the r-th M-point transform's output k' (dft_reg3).
+template <int N>
+__device__ __forceinline__ constexpr int dft_pos(int k)
+{
+	if (fft_is_pow2(N)) return brev_c(k, N);
+	return (k % 3) * (N / 3) + brev_c(k / 3, N / 3);
+}
 
 // Radix-2 DIF stages of span SPAN0, SPAN0/2, ..., 1 over v[0..N) (the full DFT has SPAN0 = N/2).
 template <typename T, int N, bool INV, int SPAN0>
@@ -68,10 +90,49 @@ __device__ __forceinline__ void dif_stages(cplx<T> (&v)[N])
 	}
 }
 
+// N = 3 M points (M a power of two, N <= 48): one radix-3 stage over the inputs M apart, the
+// twiddles W_N^(r j), then three M-point transforms in place.  Outputs at dft_pos<N>.
+template <typename T, int N, bool INV>
+__device__ __forceinline__ void dft_reg3(cplx<T> (&v)[N])
+{
+	using C = cplx<T>;
+	constexpr int M = N / 3;
+	static_assert(3 * M == N && fft_is_pow2(M) && 48 % N == 0, "3 * 2^k points, at most 48");
+	const T s60 = T(0.86602540378443864676372317075293618);  // sin(60 deg)
+	C y[3][M];
+#pragma unroll
+	for (int j = 0; j < M; ++j) {
+		const C a = v[j], b = v[j + M], c = v[j + 2 * M];
+		const C s = cadd(b, c), d = csub(b, c);
+		const C t = C{a.x - T(0.5) * s.x, a.y - T(0.5) * s.y};
+		const C r = mul_mi<INV>(C{s60 * d.x, s60 * d.y});
+		y[0][j] = cadd(a, s);
+		C y1 = cadd(t, r), y2 = csub(t, r);
+		if (j > 0) {
+			C w1 = w48<T>(j * (48 / N)), w2 = w48<T>(2 * j * (48 / N));
+			if (INV) {
+				w1 = conjc(w1);
+				w2 = conjc(w2);
+			}
+			y1 = cmul(y1, w1);
+			y2 = cmul(y2, w2);
+		}
+		y[1][j] = y1;
+		y[2][j] = y2;
+	}
+#pragma unroll
+	for (int r = 0; r < 3; ++r) {
+		if constexpr (M > 1) dif_stages<T, M, INV, M / 2>(y[r]);
+#pragma unroll
+		for (int j = 0; j < M; ++j) v[r * M + j] = y[r][j];
+	}
+}
+
 template <typename T, int N, bool INV>
 __device__ __forceinline__ void dft_reg(cplx<T> (&v)[N])
 {
-	dif_stages<T, N, INV, N / 2>(v);
+	if constexpr (fft_is_pow2(N)) dif_stages<T, N, INV, N / 2>(v);
+	else dft_reg3<T, N, INV>(v);
 }
 
 // Forward DFT of a column whose upper half v[N/2..N) is zero padding: the first DIF stage reduces
@@ -79,7 +140,11 @@ __device__ __forceinline__ void dft_reg(cplx<T> (&v)[N])
 template <typename T, int N>
 __device__ __forceinline__ void dft_reg_halfzero(cplx<T> (&v)[N])
 {
-	if constexpr (N >= 2) {
+	if constexpr (!fft_is_pow2(N)) {
+#pragma unroll
+		for (int j = N / 2; j < N; ++j) v[j] = cplx<T>{T(0), T(0)};
+		dft_reg3<T, N, false>(v);
+	} else if constexpr (N >= 2) {
 #pragma unroll
 		for (int j = 0; j < N / 2; ++j) {
 			const int q = j * (64 / N);
@@ -97,14 +162,29 @@ namespace mm {
 
 // ---- CTA-wide Stockham FFT with compile-time length and radix -----------------------------------
 // LANES independent lines of length N live in shared memory; each of the N/R threads of a line
-// performs R/Rp radix-Rp butterflies per pass (Rp = R except possibly a smaller last pass).  Pass 0
+// performs R/Rp radix-Rp butterflies per pass (Rp: fft_radix).  Pass 0
 // reads its inputs through `ld(line, k)` (global memory, with zero padding), the last pass hands
 // its outputs to `st(line, k, value)`; intermediate passes go through shared memory at
 // `SmIdx::at(line, k)`.  All strides are compile-time powers of two.
 __host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n / 2); }
-__host__ __device__ constexpr int fft_npasses(int N, int R) { return (ilog2c(N) + ilog2c(R) - 1) / ilog2c(R); }
+// Radices: a power of two takes passes of radix R and a smaller last one; N = 3 * 2^k (R = 24, or
+// N itself below 24) takes radix 8 until at most 24 points are left, which are the last pass (so
+// the factor 3 comes last and every earlier stride stays a power of two).
+__host__ __device__ constexpr int fft_npasses(int N, int R)
+{
+	if (!fft_is_pow2(N)) {
+		int p = 1;
+		for (; N > 24; N /= 8) ++p;
+		return p;
+	}
+	return (ilog2c(N) + ilog2c(R) - 1) / ilog2c(R);
+}
 __host__ __device__ constexpr int fft_radix(int N, int R, int p)
 {
+	if (!fft_is_pow2(N)) {
+		for (; p > 0; --p) N /= 8;
+		return N > 24 ? 8 : N;
+	}
 	return ilog2c(N) - p * ilog2c(R) >= ilog2c(R) ? R : (1 << (ilog2c(N) - p * ilog2c(R)));
 }
 
@@ -158,12 +238,13 @@ __device__ __forceinline__ void cta_fft_pass(cplx<T> *sm, const cplx<T> *__restr
 	using C = cplx<T>;
 	constexpr int P = fft_npasses(N, R);
 	constexpr int Rp = fft_radix(N, R, p);
-	constexpr int Ns = 1 << (p * ilog2c(R));  // product of the radices of earlier passes
+	constexpr int Ns = 1 << (p * (fft_is_pow2(N) ? ilog2c(R) : 3));  // product of the radices of earlier passes
 	constexpr int TPL = N / R;
 	constexpr int BPT = R / Rp;
 	constexpr int M = N / Rp;                  // butterflies per line, input stride
 	constexpr bool HALF = H0 && p == 0;
-	static_assert(!HALF || (!INV && BPT == 1 && Rp >= 2), "half-zero pass 0: forward, one butterfly per thread");
+	static_assert(!HALF || (!INV && Rp % 2 == 0), "half-zero pass 0: forward, an even radix");
+	static_assert(R % Rp == 0, "a thread takes whole butterflies");
 	C v[BPT][Rp];
 	if constexpr (p > 0) __syncthreads();
 #pragma unroll
@@ -194,7 +275,7 @@ __device__ __forceinline__ void cta_fft_pass(cplx<T> *sm, const cplx<T> *__restr
 		const int base = (j / Ns) * Ns * Rp + jm;
 #pragma unroll
 		for (int k = 0; k < Rp; ++k) {
-			const C val = v[u][brev<Rp>(k)];
+			const C val = v[u][dft_pos<Rp>(k)];
 			if constexpr (p == P - 1) st(line, base + k * Ns, val);
 			else sm[SmIdx::at(line, base + k * Ns)] = val;
 		}
@@ -235,6 +316,13 @@ static inline mm_status fft_reg_init()
 	}
 	MM_CUDA(cudaMemcpyToSymbol(c_w64d, d, sizeof(d)));
 	MM_CUDA(cudaMemcpyToSymbol(c_w64f, f, sizeof(f)));
+	for (int k = 0; k < 48; ++k) {
+		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / 48.0L;
+		d[k] = double2{(double)cosl(a), (double)sinl(a)};
+		f[k] = float2{(float)cosl(a), (float)sinl(a)};
+	}
+	MM_CUDA(cudaMemcpyToSymbol(c_w48d, d, 48 * sizeof(double2)));
+	MM_CUDA(cudaMemcpyToSymbol(c_w48f, f, 48 * sizeof(float2)));
 	return MM_OK;
 }
 

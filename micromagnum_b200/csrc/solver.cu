@@ -1988,7 +1988,7 @@ void free_solver(mm_solver *s)
 
 template <typename T>
 mm_status create_impl(mm_solver *s, int nmat, const mm_material *mats, const uint8_t *regions,
-                      const double *tensor, cudaStream_t st)
+                      const double *tensor, cudaStream_t st, bool keep_lengths)
 {
 	s->nmat = nmat;
 	MM_TRY(build_materials<T>(s, nmat, mats));
@@ -2015,7 +2015,7 @@ mm_status create_impl(mm_solver *s, int nmat, const mm_material *mats, const uin
 			if (r != MM_OK) { cudaFree(N); return r; }
 		}
 		const mm_status r = conv_plan_create(&s->conv, c.precision, c.nx, c.ny, c.nz, s->px, s->py, s->pz,
-		                                     tensor ? tensor : N, st);
+		                                     tensor ? tensor : N, st, keep_lengths);
 		if (N) cudaFree(N);
 		MM_TRY(r);
 	}
@@ -2051,7 +2051,8 @@ namespace mm {
 namespace {
 
 // mm_solver_create with a lower bound on the padded z length (the batch pads a single layer to
-// 2 so that every instance takes the 3-D power-of-two passes).
+// 2, and keeps the tensor's lengths as FFT lengths, so that every instance takes the 3-D
+// power-of-two passes).
 mm_status solver_create(mm_solver **out, const mm_solver_config *config, int num_materials,
                         const mm_material *materials_host, const uint8_t *regions_host,
                         const double *tensor_device, void *stream, int min_pz)
@@ -2084,8 +2085,8 @@ mm_status solver_create(mm_solver **out, const mm_solver_config *config, int num
 	s->h = c.h0;
 	cudaStream_t st = as_stream(stream);
 	const mm_status r = c.precision == MM_F64
-	                        ? create_impl<double>(s, num_materials, materials_host, regions_host, tensor_device, st)
-	                        : create_impl<float>(s, num_materials, materials_host, regions_host, tensor_device, st);
+	                        ? create_impl<double>(s, num_materials, materials_host, regions_host, tensor_device, st, min_pz > 1)
+	                        : create_impl<float>(s, num_materials, materials_host, regions_host, tensor_device, st, min_pz > 1);
 	if (r != MM_OK) {
 		free_solver(s);
 		return r;
