@@ -22,10 +22,10 @@ FftRadices fft_factor(int n)
 }
 
 // conv_f64.cu, conv_f32.cu
-mm_status conv_setup_f64(ConvPlan *p, const double *N, cudaStream_t st);
+mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
 mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st);
 int conv_fit_length_f64(int n, int e, bool z);
-mm_status conv_setup_f32(ConvPlan *p, const double *N, cudaStream_t st);
+mm_status conv_setup_f32(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
 mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st);
 int conv_fit_length_f32(int n, int e, bool z);
 
@@ -106,10 +106,11 @@ ConvPlan::~ConvPlan()
 int conv_launches(const ConvPlan *p) { return p->is2d ? 3 : 5; }
 
 mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey, int ez,
-                           const double *N, cudaStream_t st, bool keep_lengths)
+                           const double *N, cudaStream_t st, bool keep_lengths, bool octant)
 {
 	if (prec != MM_F64 && prec != MM_F32) return fail(MM_ERR_INVALID_ARGUMENT, "conv: bad precision");
-	if (nx <= 0 || ny <= 0 || nz <= 0 || ex < nx || ey < ny || ez < nz || !N)
+	if (nx <= 0 || ny <= 0 || nz <= 0 || ex < nx || ey < ny || ez < nz || !N ||
+	    (octant && (ex < 2 * nx - 1 || ey < 2 * ny - 1 || ez < 2 * nz - 1)))
 		return fail(MM_ERR_INVALID_ARGUMENT, "conv: invalid sizes or null tensor");
 	auto length = [&](int n, int e, bool z) {
 		return keep_lengths ? e : prec == MM_F64 ? conv_fit_length_f64(n, e, z) : conv_fit_length_f32(n, e, z);
@@ -142,7 +143,7 @@ mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int
 		delete p;
 		return fail(MM_ERR_UNSUPPORTED, "conv: FFT length has too many prime factors");
 	}
-	const mm_status s = prec == MM_F64 ? conv_setup_f64(p, N, st) : conv_setup_f32(p, N, st);
+	const mm_status s = prec == MM_F64 ? conv_setup_f64(p, N, octant, st) : conv_setup_f32(p, N, octant, st);
 	if (s != MM_OK) {
 		delete p;
 		return s;

@@ -45,7 +45,6 @@ struct ConvPlan {
 	int lp_x = 1;                   // complex lines (= 2 real rows) per CTA in the x passes
 	int tb_y = 1, tb_z = 1;         // columns per CTA in the y and z passes
 	size_t smem_x = 0, smem_y = 0, smem_z = 0;
-	double max_imag_rel = 0.0;      // largest |Im N^| / max |Re N^| seen at set-up
 
 	size_t spec_bytes() const;
 	~ConvPlan();
@@ -54,8 +53,13 @@ struct ConvPlan {
 // Builds the plan and the tensor spectrum from an FP64 tensor in the reference layout
 // (component fastest, then x, y, z) of padded size ex*ey*ez.  The FFT lengths of zero-padded axes are
 // the plan's choice (keep_lengths: the tensor's own, as the grouped passes need powers of two).
+// octant: N holds only the offsets >= 0 of a box without periodic axes, [nz][ny][nx][6].
 mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey,
-                           int ez, const double *N_device, cudaStream_t st, bool keep_lengths = false);
+                           int ez, const double *N_device, cudaStream_t st, bool keep_lengths = false,
+                           bool octant = false);
+
+// The tensor's octant of offsets >= 0 of a box without periodic axes, [nz][ny][nx][6] (tensor.cu).
+mm_status tensor_octant(int nx, int ny, int nz, double dx, double dy, double dz, double *N, cudaStream_t st);
 
 // H = N * (Ms[region] * M) when regions/ms_table are given (ms_table: 256 entries), else H = N * M.
 // M and H are SoA arrays of T (T = double for MM_F64, float for MM_F32).

@@ -3,7 +3,7 @@
 
 namespace mm {
 
-mm_status conv_setup_f32(ConvPlan *p, const double *N, cudaStream_t st) { return plan_setup<float>(p, N, st); }
+mm_status conv_setup_f32(ConvPlan *p, const double *N, bool octant, cudaStream_t st) { return plan_setup<float>(p, N, octant, st); }
 
 mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st)
 {

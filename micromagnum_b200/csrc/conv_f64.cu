@@ -3,7 +3,7 @@
 
 namespace mm {
 
-mm_status conv_setup_f64(ConvPlan *p, const double *N, cudaStream_t st) { return plan_setup<double>(p, N, st); }
+mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st) { return plan_setup<double>(p, N, octant, st); }
 
 mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st)
 {

@@ -20,7 +20,9 @@
 // fastest), components (xx, xy, xz, yy, yz, zz), scattered into the eight octants with the
 // parities of tensor.cpp:167-180.
 #include "mm_common.cuh"
+#include "conv.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <mutex>
@@ -31,9 +33,10 @@ namespace {
 
 constexpr int GL_MAX = 40;
 
+// Quadrature of one tent of half-width 1: 2 n (node, weight) pairs for n nodes per half, the table for
+// n starting at n (n - 1).  The weights include the tent, 1 - |node|.
 struct GLTable {
-	double *x = nullptr;  // nodes on [-1, 1], table for n starts at n(n-1)/2
-	double *w = nullptr;
+	double2 *xw = nullptr;
 };
 
 // Gauss-Legendre nodes and weights by Newton iteration on P_n (long double).
@@ -81,18 +84,20 @@ mm_status gl_table(GLTable **out)
 	std::lock_guard<std::mutex> lock(mu);
 	if ((int)tabs.size() <= dev) tabs.resize(dev + 1);
 	GLTable &tab = tabs[dev];
-	if (!tab.x) {
-		std::vector<double> hx, hw, x, w;
+	if (!tab.xw) {
+		std::vector<double> x, w;
+		std::vector<double2> h;
 		for (int n = 1; n <= GL_MAX; ++n) {
 			if (n == 1) { x = {0.0}; w = {2.0}; }
 			else gauss_legendre(n, x, w);
-			hx.insert(hx.end(), x.begin(), x.end());
-			hw.insert(hw.end(), w.begin(), w.end());
+			for (double half : {-0.5, 0.5})
+				for (int q = 0; q < n; ++q) {
+					const double u = half + 0.5 * x[q];
+					h.push_back(double2{u, 0.5 * w[q] * (1.0 - std::fabs(u))});
+				}
 		}
-		MM_CUDA(cudaMalloc(&tab.x, hx.size() * sizeof(double)));
-		MM_CUDA(cudaMalloc(&tab.w, hw.size() * sizeof(double)));
-		MM_CUDA(cudaMemcpy(tab.x, hx.data(), hx.size() * sizeof(double), cudaMemcpyHostToDevice));
-		MM_CUDA(cudaMemcpy(tab.w, hw.data(), hw.size() * sizeof(double), cudaMemcpyHostToDevice));
+		MM_CUDA(cudaMalloc(&tab.xw, h.size() * sizeof(double2)));
+		MM_CUDA(cudaMemcpy(tab.xw, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
 	}
 	*out = &tab;
 	return MM_OK;
@@ -151,7 +156,7 @@ __device__ void tensor_newell(int i, int j, int k, double dx, double dy, double 
 	for (int c = 0; c < 6; ++c) v[c] = pref * acc[c];
 }
 
-__device__ int gl_order(double D, double halfwidth)
+__host__ __device__ inline int gl_order(double D, double halfwidth)
 {
 	const double r = D / halfwidth;
 	const double rho = r + sqrt(r * r + 1.0);
@@ -161,10 +166,9 @@ __device__ int gl_order(double D, double halfwidth)
 	return n < 3.0 ? 3 : (n > GL_MAX ? GL_MAX + 1 : (int)n);
 }
 
-// Negated tensor at offset (i, j, k) by quadrature; returns false if the orders needed exceed
-// the table (the caller then uses Newell's formulas).
-__device__ bool tensor_quad(int i, int j, int k, double dx, double dy, double dz, const double *glx,
-                            const double *glw, double *v)
+// Nodes per half tent along each axis for offset (i, j, k); false if they exceed the table (the
+// caller then uses Newell's formulas).
+__host__ __device__ inline bool quad_orders(int i, int j, int k, double dx, double dy, double dz, int (&n)[3])
 {
 	const double X[3] = {i * dx, j * dy, k * dz};
 	const double a[3] = {dx, dy, dz};
@@ -174,72 +178,157 @@ __device__ bool tensor_quad(int i, int j, int k, double dx, double dy, double dz
 		g2 += g * g;
 	}
 	const double D = sqrt(g2);
-	int n[3];
 	for (int c = 0; c < 3; ++c) {
 		n[c] = gl_order(D, 0.5 * a[c]);
 		if (n[c] > GL_MAX) return false;
 	}
-	const double *xs[3], *ws[3];
-	for (int c = 0; c < 3; ++c) {
-		xs[c] = glx + n[c] * (n[c] - 1) / 2;
-		ws[c] = glw + n[c] * (n[c] - 1) / 2;
-	}
-	double acc[6] = {0, 0, 0, 0, 0, 0};
-	// u_c in [-a_c, 0] and [0, a_c]: u = (s - 1 + ... ) mapped per half, tent weight (a - |u|)
-	for (int hz = 0; hz < 2; ++hz)
-		for (int qz = 0; qz < n[2]; ++qz) {
-			const double uz = (hz ? 0.5 : -0.5) * a[2] + 0.5 * a[2] * xs[2][qz];
-			const double wz = 0.5 * a[2] * ws[2][qz] * (a[2] - fabs(uz));
-			const double rz = X[2] + uz;
-			for (int hy = 0; hy < 2; ++hy)
-				for (int qy = 0; qy < n[1]; ++qy) {
-					const double uy = (hy ? 0.5 : -0.5) * a[1] + 0.5 * a[1] * xs[1][qy];
-					const double wyz = wz * 0.5 * a[1] * ws[1][qy] * (a[1] - fabs(uy));
-					const double ry = X[1] + uy;
-					const double ryz2 = ry * ry + rz * rz;
-					double s_xx = 0, s_xy = 0, s_xz = 0, s_yy = 0, s_yz = 0, s_zz = 0;
-					for (int hx = 0; hx < 2; ++hx)
-						for (int qx = 0; qx < n[0]; ++qx) {
-							const double ux = (hx ? 0.5 : -0.5) * a[0] + 0.5 * a[0] * xs[0][qx];
-							const double wx = 0.5 * a[0] * ws[0][qx] * (a[0] - fabs(ux));
-							const double rx = X[0] + ux;
-							const double r2 = rx * rx + ryz2;
-							const double ir = rsqrt(r2);
-							const double ir3 = ir * ir * ir;
-							const double w3 = wx * ir3;
-							const double w5 = 3.0 * w3 / r2;
-							s_xx += w3 - w5 * rx * rx;
-							s_yy += w3 - w5 * ry * ry;
-							s_zz += w3 - w5 * rz * rz;
-							s_xy -= w5 * rx * ry;
-							s_xz -= w5 * rx * rz;
-							s_yz -= w5 * ry * rz;
-						}
-					acc[0] += wyz * s_xx;
-					acc[1] += wyz * s_xy;
-					acc[2] += wyz * s_xz;
-					acc[3] += wyz * s_yy;
-					acc[4] += wyz * s_yz;
-					acc[5] += wyz * s_zz;
-				}
-		}
-	const double pref = -1.0 / (4.0 * PI * dx * dy * dz);
-	for (int c = 0; c < 6; ++c) v[c] = pref * acc[c];
 	return true;
 }
 
+// Quadrature sums of offset (i, j, k) over the (y, z) node pairs first, first + step, ...: the
+// negated tensor without its factor V / 4 pi.  Along x four moments of the row are summed (of
+// r^-3 and 3 r^-5 with rx^0, rx^1, rx^2), from which the six components of the row follow.
+__device__ __forceinline__ void quad_sums(int i, int j, int k, double dx, double dy, double dz, const int (&n)[3],
+                                          const double2 *__restrict__ gl, int first, int step, double (&acc)[6])
+{
+	const double X = i * dx, Y = j * dy, Z = k * dz;
+	const double2 *gx = gl + n[0] * (n[0] - 1), *gy = gl + n[1] * (n[1] - 1), *gz = gl + n[2] * (n[2] - 1);
+	const int nx = 2 * n[0], ny = 2 * n[1], rows = ny * 2 * n[2];
+	for (int c = 0; c < 6; ++c) acc[c] = 0.0;
+	for (int row = first; row < rows; row += step) {
+		const int qz = row / ny, qy = row - qz * ny;
+		const double2 ny2 = gy[qy], nz2 = gz[qz];
+		const double ry = Y + ny2.x * dy, rz = Z + nz2.x * dz, wyz = ny2.y * nz2.y;
+		const double ryz2 = ry * ry + rz * rz;
+		double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+#pragma unroll 4
+		for (int qx = 0; qx < nx; ++qx) {
+			const double2 nd = gx[qx];
+			const double rx = X + nd.x * dx;
+			const double r2 = rx * rx + ryz2;
+			const double ir = rsqrt(r2);
+			const double ir2 = ir * ir;
+			const double w3 = nd.y * (ir2 * ir);
+			const double w5 = 3.0 * w3 * ir2, w5x = w5 * rx;
+			a0 += w3;
+			a1 += w5;
+			a2 += w5x;
+			a3 += w5x * rx;
+		}
+		acc[0] += wyz * (a0 - a3);
+		acc[1] -= wyz * ry * a2;
+		acc[2] -= wyz * rz * a2;
+		acc[3] += wyz * (a0 - ry * ry * a1);
+		acc[4] -= wyz * (ry * rz * a1);
+		acc[5] += wyz * (a0 - rz * rz * a1);
+	}
+}
+
+// The offsets next to the origin need high orders (27,000 points two cells away, 1,000 to 1,700 for
+// most of a mesh), and one thread per offset made them the kernel's whole time (7.6 ms at 240x120x10
+// cells, FP64, of which 0.6 ms are the other offsets).  So the box of offsets that need more than
+// NEAR_POINTS points is computed first, a block per offset, and looked up by the kernels that follow.
+constexpr int NEAR_POINTS = 2000, NEAR_MAX = 1 << 16, NEAR_THREADS = 128;
+
+struct NearBox {
+	int x = 0, y = 0, z = 0;    // offsets i < x, j < y, k < z
+	int lx = 0, ly = 0;         // layout: six values at v + 6 ((k ly + j) lx + i)
+	double *v = nullptr;
+	__host__ __device__ double *at(int i, int j, int k) const { return v + 6 * (((size_t)k * ly + j) * lx + i); }
+};
+
+__global__ void __launch_bounds__(NEAR_THREADS) k_tensor_near(NearBox nb, double dx, double dy, double dz,
+                                                              const double2 *__restrict__ gl)
+{
+	const int q = blockIdx.x, i = q % nb.x, j = q / nb.x % nb.y, k = q / (nb.x * nb.y);
+	double *out = nb.at(i, j, k);
+	int n[3];
+	if ((i <= 1 && j <= 1 && k <= 1) || !quad_orders(i, j, k, dx, dy, dz, n)) {
+		if (threadIdx.x == 0) tensor_newell(i, j, k, dx, dy, dz, out);
+		return;
+	}
+	double acc[6];
+	quad_sums(i, j, k, dx, dy, dz, n, gl, threadIdx.x, NEAR_THREADS, acc);
+	__shared__ double red[6][NEAR_THREADS / 32];
+	for (int c = 0; c < 6; ++c) {
+		const double w = warp_sum(acc[c]);
+		if ((threadIdx.x & 31) == 0) red[c][threadIdx.x >> 5] = w;
+	}
+	__syncthreads();
+	if (threadIdx.x < 6) {
+		double sum = 0;
+		for (int w = 0; w < NEAR_THREADS / 32; ++w) sum += red[threadIdx.x][w];
+		out[threadIdx.x] = -dx * dy * dz / (4.0 * PI) * sum;
+	}
+}
+
+// Host: the extents of the near box for offsets up to nx, ny, nz (not included).
+void near_extents(int nx, int ny, int nz, double dx, double dy, double dz, NearBox &nb)
+{
+	const int lim[3] = {nx, ny, nz};
+	int ext[3];
+	const long long most = 8LL * GL_MAX * GL_MAX * GL_MAX;
+	for (long long points = NEAR_POINTS;; points *= 2) {
+		for (int a = 0; a < 3; ++a) {
+			// along the axis: the first offset that needs few points (the orders fall with distance)
+			int lo = std::min(2, lim[a]), hi = points <= most ? lim[a] : lo;
+			while (lo < hi) {
+				const int mid = lo + (hi - lo) / 2;
+				int n[3];
+				const bool few = quad_orders(a == 0 ? mid : 0, a == 1 ? mid : 0, a == 2 ? mid : 0, dx, dy, dz, n) &&
+				                 8LL * n[0] * n[1] * n[2] <= points;
+				if (few) hi = mid;
+				else lo = mid + 1;
+			}
+			ext[a] = lo;
+		}
+		if ((long long)ext[0] * ext[1] * ext[2] <= NEAR_MAX) break;  // (a box of two cells a side at the last)
+	}
+	nb.x = ext[0];
+	nb.y = ext[1];
+	nb.z = ext[2];
+}
+
+mm_status tensor_near(const NearBox &nb, double dx, double dy, double dz, const double2 *gl, cudaStream_t st)
+{
+	k_tensor_near<<<nb.x * nb.y * nb.z, NEAR_THREADS, 0, st>>>(nb, dx, dy, dz, gl);
+	return after_launch("k_tensor_near");
+}
+
+// Negated tensor (xx, xy, xz, yy, yz, zz) at offset (i, j, k) >= 0.
+__device__ __forceinline__ void tensor_at(int i, int j, int k, double dx, double dy, double dz, const NearBox &nb,
+                                          const double2 *__restrict__ gl, double (&v)[6])
+{
+	if (i < nb.x && j < nb.y && k < nb.z) {
+		const double *t = nb.at(i, j, k);
+		for (int c = 0; c < 6; ++c) v[c] = t[c];
+		return;
+	}
+	int n[3];
+	if (!quad_orders(i, j, k, dx, dy, dz, n)) {
+		tensor_newell(i, j, k, dx, dy, dz, v);
+		return;
+	}
+	quad_sums(i, j, k, dx, dy, dz, n, gl, 0, 1, v);
+	const double f = -dx * dy * dz / (4.0 * PI);
+	for (int c = 0; c < 6; ++c) v[c] *= f;
+}
+
+// OCTANT: offsets >= 0 only, [nz][ny][nx][6] (ex = nx, ey = ny); else the padded layout, every octant.
+template <bool OCTANT>
 __global__ void __launch_bounds__(128) k_demag_tensor(int nx, int ny, int nz, double dx, double dy,
-                                                      double dz, int ex, int ey, int ez,
-                                                      const double *__restrict__ glx,
-                                                      const double *__restrict__ glw,
-                                                      double *__restrict__ out)
+                                                      double dz, int ex, int ey, int ez, NearBox nb,
+                                                      const double2 *__restrict__ gl, double *out)
 {
 	const size_t cnt = (size_t)nx * ny * nz;
 	for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < cnt; q += (size_t)gridDim.x * blockDim.x) {
 		const int i = (int)(q % nx), j = (int)((q / nx) % ny), k = (int)(q / ((size_t)nx * ny));
 		double v[6];
-		const bool touching = i <= 1 && j <= 1 && k <= 1;
-		if (touching || !tensor_quad(i, j, k, dx, dy, dz, glx, glw, v)) tensor_newell(i, j, k, dx, dy, dz, v);
+		tensor_at(i, j, k, dx, dy, dz, nb, gl, v);
+		if (OCTANT) {
+			for (int c = 0; c < 6; ++c) out[6 * q + c] = v[c];
+			continue;
+		}
 		for (int o = -1; o <= 1; o += 2)
 			for (int p = -1; p <= 1; p += 2)
 				for (int r = -1; r <= 1; r += 2) {
@@ -254,6 +343,26 @@ __global__ void __launch_bounds__(128) k_demag_tensor(int nx, int ny, int nz, do
 					d[5] = v[5];
 				}
 	}
+}
+
+// The near box goes to its place in the output, where the next kernel's thread of the same offset
+// reads it (no other thread writes offsets i < nx, j < ny, k < nz).
+template <bool OCTANT>
+mm_status tensor_run(int nx, int ny, int nz, double dx, double dy, double dz, int ex, int ey, int ez, double *out,
+                     cudaStream_t st)
+{
+	GLTable *gl = nullptr;
+	MM_TRY(gl_table(&gl));
+	NearBox nb;
+	near_extents(nx, ny, nz, dx, dy, dz, nb);
+	nb.lx = ex;
+	nb.ly = ey;
+	nb.v = out;
+	MM_TRY(tensor_near(nb, dx, dy, dz, gl->xw, st));
+	const size_t want = ((size_t)nx * ny * nz + 127) / 128;
+	const int grid = (int)(want < 65535u * 16 ? want : 65535u * 16);
+	k_demag_tensor<OCTANT><<<grid, 128, 0, st>>>(nx, ny, nz, dx, dy, dz, ex, ey, ez, nb, gl->xw, out);
+	return after_launch("k_demag_tensor");
 }
 
 // ---- periodic boundaries (tensor.cpp:35-165 with demag_tensor.cpp:116-186) --------------------
@@ -387,9 +496,8 @@ __device__ void corner_tail(double P[3], int A, int B, double LA, double LB, dou
 // Sum over images of the negated tensor of source offset (i, j, k), halved for each coordinate
 // at zero displacement, plus the far images (tails); out[6] per source offset.
 __global__ void __launch_bounds__(128) k_tensor_images(int nx, int ny, int nz, double dx, double dy, double dz,
-                                                       int Rx, int Ry, int Rz, int tails,
-                                                       const double *__restrict__ glx,
-                                                       const double *__restrict__ glw, double *__restrict__ out)
+                                                       int Rx, int Ry, int Rz, int tails, NearBox nb,
+                                                       const double2 *__restrict__ gl, double *__restrict__ out)
 {
 	const size_t cnt = (size_t)nx * ny * nz;
 	const int n3[3] = {nx, ny, nz}, R3[3] = {Rx, Ry, Rz};
@@ -404,8 +512,7 @@ __global__ void __launch_bounds__(128) k_tensor_images(int nx, int ny, int nz, d
 					const int I = ijk[0] + rx * nx, J = ijk[1] + ry * ny, K = ijk[2] + rz * nz;
 					const double w = (I == 0 ? 0.5 : 1.0) * (J == 0 ? 0.5 : 1.0) * (K == 0 ? 0.5 : 1.0);
 					double v[6];
-					const bool touching = I <= 1 && J <= 1 && K <= 1;
-					if (touching || !tensor_quad(I, J, K, dx, dy, dz, glx, glw, v)) tensor_newell(I, J, K, dx, dy, dz, v);
+					tensor_at(I, J, K, dx, dy, dz, nb, gl, v);
 					for (int c = 0; c < 6; ++c) S[c] += w * v[c];
 				}
 		if (tails) {
@@ -482,6 +589,12 @@ __global__ void __launch_bounds__(128) k_tensor_gather(int nx, int ny, int nz, i
 }
 
 } // namespace
+
+mm_status tensor_octant(int nx, int ny, int nz, double dx, double dy, double dz, double *N, cudaStream_t st)
+{
+	return tensor_run<true>(nx, ny, nz, dx, dy, dz, nx, ny, nz, N, st);
+}
+
 } // namespace mm
 
 using namespace mm;
@@ -522,14 +635,8 @@ MM_API mm_status mm_demag_tensor(int nx, int ny, int nz, double dx, double dy, d
 		return fail(MM_ERR_UNSUPPORTED,
 		            "mm_demag_tensor: padded sizes below 2n-1 (periodic boundaries) are not supported");
 	cudaStream_t st = as_stream(stream);
-	GLTable *gl = nullptr;
-	MM_TRY(gl_table(&gl));
 	MM_CUDA(cudaMemsetAsync(N_out, 0, sizeof(double) * 6 * (size_t)ex * ey * ez, st));
-	const size_t cnt = (size_t)nx * ny * nz;
-	const size_t want = (cnt + 127) / 128;
-	const int grid = (int)(want < 65535u * 16 ? want : 65535u * 16);
-	k_demag_tensor<<<grid, 128, 0, st>>>(nx, ny, nz, dx, dy, dz, ex, ey, ez, gl->x, gl->w, N_out);
-	return after_launch("k_demag_tensor");
+	return tensor_run<false>(nx, ny, nz, dx, dy, dz, ex, ey, ez, N_out, st);
 }
 
 MM_API mm_status mm_demag_tensor_periodic(int nx, int ny, int nz, double dx, double dy, double dz, int pbc_x,
@@ -548,14 +655,23 @@ MM_API mm_status mm_demag_tensor_periodic(int nx, int ny, int nz, double dx, dou
 	GLTable *gl = nullptr;
 	MM_TRY(gl_table(&gl));
 	const size_t cnt = (size_t)nx * ny * nz;
-	double *S = nullptr;
-	MM_CUDA(cudaMallocAsync(&S, 6 * cnt * sizeof(double), st));
 	const char *off = std::getenv("MAGNUM_DEMAG_NO_INFINITY_CORRECTION");  // tensor.cpp:45
 	const int Rx = pbc_x ? repeat : 1, Ry = pbc_y ? repeat : 1, Rz = pbc_z ? repeat : 1;
+	NearBox nb;  // (the images' offsets run past the mesh)
+	auto reach = [](int n, int R) { return (int)std::min<long long>((long long)n * R, 1 << 30); };
+	near_extents(reach(nx, Rx), reach(ny, Ry), reach(nz, Rz), dx, dy, dz, nb);
+	nb.lx = nb.x;
+	nb.ly = nb.y;
+	double *S = nullptr;  // the source offsets' sums, then the near box
+	MM_CUDA(cudaMallocAsync(&S, 6 * (cnt + (size_t)nb.x * nb.y * nb.z) * sizeof(double), st));
+	nb.v = S + 6 * cnt;
+	mm_status r = tensor_near(nb, dx, dy, dz, gl->xw, st);
 	const size_t want = (cnt + 127) / 128;
-	k_tensor_images<<<(int)(want < 65535u * 16 ? want : 65535u * 16), 128, 0, st>>>(
-	    nx, ny, nz, dx, dy, dz, Rx, Ry, Rz, off ? 0 : 1, gl->x, gl->w, S);
-	mm_status r = after_launch("k_tensor_images");
+	if (r == MM_OK) {
+		k_tensor_images<<<(int)(want < 65535u * 16 ? want : 65535u * 16), 128, 0, st>>>(
+		    nx, ny, nz, dx, dy, dz, Rx, Ry, Rz, off ? 0 : 1, nb, gl->xw, S);
+		r = after_launch("k_tensor_images");
+	}
 	if (r == MM_OK) {
 		const size_t out = (size_t)ex * ey * ez, w2 = (out + 127) / 128;
 		k_tensor_gather<<<(int)(w2 < 65535u * 16 ? w2 : 65535u * 16), 128, 0, st>>>(nx, ny, nz, ex, ey, ez, S, N_out);
