@@ -1,8 +1,8 @@
 // Register-resident FFT building blocks for power-of-two lengths (included by conv.cu only).
 //
 // dft_reg<T, N, INV>: an N-point DFT (N = 1..64) held entirely in one thread's registers,
-// radix-2 decimation in frequency (after one radix-3 stage for N = 3 * 2^k <= 48), fully unrolled,
-// output k in register dft_pos<N>(k).  Its twiddles W_64^q = exp(-2 pi i q / 64) live in a __constant__ table that every
+// radix-4 decimation in frequency (a radix-2 stage last where 4 does not divide, after one radix-3
+// stage for N = 3 * 2^k <= 48), fully unrolled, output k in register dft_pos<N>(k).  Its twiddles W_64^q = exp(-2 pi i q / 64) live in a __constant__ table that every
 // lane reads at the same compile-time index (a broadcast).
 //
 // Longer transforms (N = N1 * N2 <= 4096) use the four-step decomposition within a CTA:
@@ -62,30 +62,47 @@ __device__ __forceinline__ constexpr int dft_pos(int k)
 	return (k % 3) * (N / 3) + brev_c(k / 3, N / 3);
 }
 
-// Radix-2 DIF stages of span SPAN0, SPAN0/2, ..., 1 over v[0..N) (the full DFT has SPAN0 = N/2).
+// v W_64^q (conjugated for the inverse), q a compile-time constant after unrolling.
+template <typename T, bool INV>
+__device__ __forceinline__ cplx<T> mul_w64(cplx<T> v, int q)
+{
+	if (q == 0) return v;
+	if (q == 16) return mul_mi<INV>(v);
+	cplx<T> w = w64<T>(q);
+	if (INV) w = conjc(w);
+	return cmul(v, w);
+}
+
+// Decimation-in-frequency stages over v[0..N): a radix-4 stage stands for the radix-2 stages of spans
+// SPAN0 and SPAN0/2 (and leaves its outputs where they would), so a value passes one twiddle
+// multiplication where two radix-2 stages have two (8 instead of 10 in a 16-point transform, and the
+// smaller rounding error); SPAN0 = N/2 is the full transform.
 template <typename T, int N, bool INV, int SPAN0>
 __device__ __forceinline__ void dif_stages(cplx<T> (&v)[N])
 {
 	using C = cplx<T>;
+	if constexpr (SPAN0 >= 2) {
+		constexpr int Q = SPAN0 / 2;  // a butterfly's inputs are Q apart, its transform has 4 Q points
 #pragma unroll
-	for (int span = SPAN0; span >= 1; span >>= 1) {
+		for (int b = 0; b < N; b += 4 * Q) {
 #pragma unroll
-		for (int b = 0; b < N; b += 2 * span) {
-#pragma unroll
-			for (int j = 0; j < span; ++j) {
-				const C a = v[b + j], c = v[b + j + span];
-				v[b + j] = cadd(a, c);
-				C d = csub(a, c);
-				const int q = j * (64 / (2 * span));  // W_{2 span}^j = W_64^q
-				if (q == 16) {
-					d = mul_mi<INV>(d);
-				} else if (q != 0) {
-					C w = w64<T>(q);
-					if (INV) w = conjc(w);
-					d = cmul(d, w);
-				}
-				v[b + j + span] = d;
+			for (int j = 0; j < Q; ++j) {
+				const C x0 = v[b + j], x1 = v[b + j + Q], x2 = v[b + j + 2 * Q], x3 = v[b + j + 3 * Q];
+				const C s0 = cadd(x0, x2), d0 = csub(x0, x2), s1 = cadd(x1, x3), d1 = mul_mi<INV>(csub(x1, x3));
+				const int q = j * (64 / (4 * Q));  // W_4Q^j = W_64^q
+				v[b + j] = cadd(s0, s1);
+				v[b + j + Q] = mul_w64<T, INV>(csub(s0, s1), 2 * q);
+				v[b + j + 2 * Q] = mul_w64<T, INV>(cadd(d0, d1), q);
+				v[b + j + 3 * Q] = mul_w64<T, INV>(csub(d0, d1), 3 * q);
 			}
+		}
+		if constexpr (Q >= 2) dif_stages<T, N, INV, Q / 2>(v);
+	} else if constexpr (SPAN0 == 1) {
+#pragma unroll
+		for (int b = 0; b < N; b += 2) {
+			const C a = v[b], c = v[b + 1];
+			v[b] = cadd(a, c);
+			v[b + 1] = csub(a, c);
 		}
 	}
 }
@@ -135,24 +152,30 @@ __device__ __forceinline__ void dft_reg(cplx<T> (&v)[N])
 	else dft_reg3<T, N, INV>(v);
 }
 
-// Forward DFT of a column whose upper half v[N/2..N) is zero padding: the first DIF stage reduces
-// to v[j + N/2] = v[j] W_N^j.  Output in bit-reversed order, like dft_reg.
+// Forward DFT of a column whose upper half v[N/2..N) is zero padding: the first stage's butterflies
+// have two inputs.  Output at dft_pos<N>, like dft_reg.
 template <typename T, int N>
 __device__ __forceinline__ void dft_reg_halfzero(cplx<T> (&v)[N])
 {
+	using C = cplx<T>;
 	if constexpr (!fft_is_pow2(N)) {
 #pragma unroll
-		for (int j = N / 2; j < N; ++j) v[j] = cplx<T>{T(0), T(0)};
+		for (int j = N / 2; j < N; ++j) v[j] = C{T(0), T(0)};
 		dft_reg3<T, N, false>(v);
-	} else if constexpr (N >= 2) {
+	} else if constexpr (N >= 4) {
+		constexpr int Q = N / 4;
 #pragma unroll
-		for (int j = 0; j < N / 2; ++j) {
+		for (int j = 0; j < Q; ++j) {
+			const C x0 = v[j], x1 = v[j + Q], r1 = mul_mi<false>(x1);
 			const int q = j * (64 / N);
-			if (q == 0) v[j + N / 2] = v[j];
-			else if (q == 16) v[j + N / 2] = mul_mi<false>(v[j]);
-			else v[j + N / 2] = cmul(v[j], w64<T>(q));
+			v[j] = cadd(x0, x1);
+			v[j + Q] = mul_w64<T, false>(csub(x0, x1), 2 * q);
+			v[j + 2 * Q] = mul_w64<T, false>(cadd(x0, r1), q);
+			v[j + 3 * Q] = mul_w64<T, false>(csub(x0, r1), 3 * q);
 		}
-		dif_stages<T, N, false, N / 4>(v);
+		if constexpr (Q >= 2) dif_stages<T, N, false, Q / 2>(v);
+	} else if constexpr (N == 2) {
+		v[1] = v[0];
 	}
 }
 
