@@ -8,7 +8,6 @@
 #include <string>
 #include <atomic>
 #include <mutex>
-#include <utility>
 
 #include "../../include/mmb200.h"
 
@@ -63,33 +62,6 @@ struct ProfToken {
 bool profiling_on();
 ProfToken prof_begin(cudaStream_t st);
 void prof_end(ProfToken tok, const char *name, double bytes, cudaStream_t st);
-
-// ---- programmatic dependent launch ------------------------------------------------------------------
-// The passes of a stage are short and each needs all of the one before.  Launched by launch_pdl, a
-// kernel's CTAs may start while its predecessor still runs: they load what no kernel of the chain writes
-// (twiddles, the Ms table, their own barriers) and stop at pdl_wait() until the predecessor has
-// completed and its writes are visible.  Every kernel launched this way calls pdl_wait() before its
-// first access to anything else, in every thread, so completion is transitive along the chain.
-// pdl_trigger() lets the successor's CTAs start once all CTAs of this grid have got that far.
-// @PDL@
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <class... P, class... A>
-inline void launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args)
-{
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	at[0].val.programmaticStreamSerializationAllowed = 1;
-	cudaLaunchConfig_t c{};
-	c.gridDim = grid;
-	c.blockDim = block;
-	c.dynamicSmemBytes = smem;
-	c.stream = st;
-	c.attrs = at;
-	c.numAttrs = 1;
-	cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);  // (a failure is the caller's after_launch's)
-}
 
 // ---- number of SMs of the current device (grid sizing) -------------------------------------------
 int num_sms();
