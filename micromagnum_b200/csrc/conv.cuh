@@ -80,7 +80,7 @@ struct ConvGroupMember {
 	const void *M[4];
 	void *H[2];
 	const uint8_t *reg;
-	const void *ms_tab;  // 256 entries
+	const void *ms_tab;  // 256 entries (reg NULL: only entry 0 is read, for every cell)
 	const int *flags;    // device run flags, NULL: always run
 };
 mm_status conv_group_create(ConvGroup **out, const ConvGroupMember *members, int count, cudaStream_t st);

@@ -777,7 +777,7 @@ mm_status group_create(ConvGroup *g, const ConvGroupMember *m, int count, cudaSt
 		d.reg = m[i].reg;
 		d.ms_tab = (const T *)m[i].ms_tab;
 		d.flags = nullptr;  // the autotuner runs every member; the real flags are set below
-		if (!d.reg || !d.ms_tab || !d.H[0]) return fail(MM_ERR_INVALID_ARGUMENT, "conv group: member without regions or output");
+		if (!d.ms_tab || !d.H[0]) return fail(MM_ERR_INVALID_ARGUMENT, "conv group: member without Ms table or output");
 		d.nx = p->nx; d.ny = p->ny; d.nz = p->nz; d.py = p->py; d.hx = p->hx; d.lx = p->lx; d.qy = p->qy; d.qz = p->qz;
 		d.tensor_t = nullptr;
 		lists[{0, p->px}].push_back(i);
