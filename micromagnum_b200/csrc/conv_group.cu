@@ -764,6 +764,10 @@ mm_status group_create(ConvGroup *g, const ConvGroupMember *m, int count, cudaSt
 		ConvPlan *p = m[i].plan;
 		if (!p || p->prec != g->prec || p->is2d || !p->fast_x || !p->fast_y || !p->reg_z)
 			return fail(MM_ERR_UNSUPPORTED, "conv group: every member needs power-of-two 3-D padding with a register z pass");
+		// (the lengths of MM_FS_SWITCH, which the grouped passes are instantiated for)
+		const int most = sizeof(T) == 4 ? 2048 : 1024;
+		if (p->px > most || p->py > most || !fft_is_pow2(p->px) || !fft_is_pow2(p->py) || !fft_is_pow2(p->pz))
+			return fail(MM_ERR_UNSUPPORTED, "conv group: a member's padded lengths are beyond the grouped passes");
 		if (2 * p->nx > p->px || 2 * p->ny > p->py || 2 * p->nz > p->pz)
 			return fail(MM_ERR_UNSUPPORTED, "conv group: every member needs zero padding to at least twice its size");
 		GDesc<T> &d = h[i];
