@@ -50,6 +50,39 @@ mm_status scalar_scratch(ScalarScratch **out)
 	return MM_OK;
 }
 
+mm_status scalar_result(ScalarResult *out)
+{
+	struct Ring {
+		ScalarSlot *slots = nullptr;
+		double *host = nullptr;
+		unsigned next = 0;
+	};
+	static std::mutex mu;
+	static std::vector<Ring> rings;
+	int dev = 0;
+	MM_CUDA(cudaGetDevice(&dev));
+	std::lock_guard<std::mutex> lock(mu);
+	if ((int)rings.size() <= dev) rings.resize(dev + 1);
+	Ring &r = rings[dev];
+	if (!r.host) {
+		ScalarSlot *slots = nullptr;
+		MM_CUDA(cudaMalloc(&slots, SCALAR_SLOTS * sizeof(ScalarSlot)));
+		MM_CUDA(cudaMemset(slots, 0, SCALAR_SLOTS * sizeof(ScalarSlot)));
+		MM_CUDA(cudaStreamSynchronize(0));  // (zeroed before a kernel of any stream can use them)
+		const mm_status s = cuda_status(cudaMallocHost(&r.host, SCALAR_SLOTS * sizeof(double)), "cudaMallocHost");
+		if (s != MM_OK) {
+			cudaFree(slots);
+			r.host = nullptr;
+			return s;
+		}
+		r.slots = slots;
+	}
+	out->slot = r.slots + r.next;
+	out->host = r.host + r.next;
+	r.next = (r.next + 1) % SCALAR_SLOTS;
+	return MM_OK;
+}
+
 // ---- profiler ------------------------------------------------------------------------------------
 namespace {
 struct ProfRecord {

@@ -180,6 +180,46 @@ __device__ __forceinline__ void block_sum_to(double *out, double v)
 	}
 }
 
+// A scalar result that a grid of 1-D blocks reduces and hands to the host by itself: the last block to
+// finish writes the total to pinned host memory and leaves the accumulator zero for the next call, so a
+// call is one kernel and one wait.  (With a memset before and a copy after the kernel, one right-hand side
+// and error norm through the magneto calls took 235 us at 160x100x4 cells, FP64, against 220.)
+struct ScalarSlot {
+	double acc;       // zero between calls
+	unsigned blocks;  // blocks that have added their part; zero between calls
+	unsigned pad;
+};
+// Called by thread 0 of each block after its atomic update of slot->acc.
+__device__ __forceinline__ void scalar_finish(ScalarSlot *slot, double *host)
+{
+	__threadfence();
+	if (atomicAdd(&slot->blocks, 1u) + 1 == gridDim.x) {
+		const unsigned long long r = atomicExch(reinterpret_cast<unsigned long long *>(&slot->acc), 0ull);
+		slot->blocks = 0;
+		*host = __longlong_as_double((long long)r);
+		__threadfence_system();
+	}
+}
+template <typename T>
+__device__ __forceinline__ void grid_max_to_host(ScalarSlot *slot, double *host, T v)
+{
+	block_max_to(&slot->acc, v);
+	if (threadIdx.x == 0) scalar_finish(slot, host);
+}
+__device__ __forceinline__ void grid_sum_to_host(ScalarSlot *slot, double *host, double v)
+{
+	block_sum_to(&slot->acc, v);
+	if (threadIdx.x == 0) scalar_finish(slot, host);
+}
+// The next slot of the device's ring (a slot comes up again after SCALAR_SLOTS further calls, each of which
+// waits for its result: that many host threads may be in such calls at once).
+constexpr int SCALAR_SLOTS = 256;
+struct ScalarResult {
+	ScalarSlot *slot = nullptr;
+	double *host = nullptr;
+};
+mm_status scalar_result(ScalarResult *out);
+
 // Serialises, across host threads, stream captures of the batch rounds against calls that can
 // synchronise the whole device or allocate (instance set-up and tear-down): a device-wide
 // synchronisation while another thread captures would invalidate that capture.

@@ -26,7 +26,7 @@ template <typename T, bool PX, bool PY, bool PZ>
 __global__ void __launch_bounds__(TPB) k_exchange(int nx, int ny, int nz, double wx, double wy,
                                                   double wz, const T *__restrict__ Ms,
                                                   const T *__restrict__ A, const T *__restrict__ M,
-                                                  T *__restrict__ H, double *energy)
+                                                  T *__restrict__ H, ScalarResult energy)
 {
 	const size_t n = (size_t)nx * ny * nz;
 	const size_t nxy = (size_t)nx * ny;
@@ -41,29 +41,34 @@ __global__ void __launch_bounds__(TPB) k_exchange(int nx, int ny, int nz, double
 			store3(H, i, n, v3<T>(0, 0, 0));
 			continue;
 		}
+		// the neighbours' Ms and M are all loaded (the cell itself in place of a missing neighbour) before
+		// the first is used, and those that do not count are selected away: behind branches each waited
+		// for the one before
+		const size_t off[6] = {x > 0 ? i - 1 : PX ? i + nx - 1 : i,        x < nx - 1 ? i + 1 : PX ? i - (nx - 1) : i,
+		                       y > 0 ? i - nx : PY ? i + nxy - nx : i,     y < ny - 1 ? i + nx : PY ? i - (nxy - nx) : i,
+		                       z > 0 ? i - nxy : PZ ? i + n - nxy : i,     z < nz - 1 ? i + nxy : PZ ? i - (n - nxy) : i};
+		const bool has[6] = {x > 0 || PX, x < nx - 1 || PX, y > 0 || PY, y < ny - 1 || PY, z > 0 || PZ, z < nz - 1 || PZ};
+		T msj[6];
+		V3<T> Mj[6];
+#pragma unroll
+		for (int q = 0; q < 6; ++q) msj[q] = Ms[off[q]];
+#pragma unroll
+		for (int q = 0; q < 6; ++q) Mj[q] = load3(M, off[q], n);
 		const V3<T> Mi = load3(M, i, n);
 		const V3<T> mi = scale_rn(T(1) / ms, Mi);
+		const T W[6] = {(T)wx, (T)wx, (T)wy, (T)wy, (T)wz, (T)wz};
 		V3<T> sum = v3<T>(0, 0, 0);
-		auto add = [&](size_t j, T w) {
-			const T msj = Ms[j];
-			if (msj != T(0)) {
-				const V3<T> mj = scale_rn(T(1) / msj, load3(M, j, n));
-				sum = sum + w * (mj - mi);
-			}
-		};
-		const T Wx = (T)wx, Wy = (T)wy, Wz = (T)wz;
-		if (x > 0) add(i - 1, Wx); else if (PX) add(i + nx - 1, Wx);
-		if (x < nx - 1) add(i + 1, Wx); else if (PX) add(i - (nx - 1), Wx);
-		if (y > 0) add(i - nx, Wy); else if (PY) add(i + nxy - nx, Wy);
-		if (y < ny - 1) add(i + nx, Wy); else if (PY) add(i - (nxy - nx), Wy);
-		if (z > 0) add(i - nxy, Wz); else if (PZ) add(i + n - nxy, Wz);
-		if (z < nz - 1) add(i + nxy, Wz); else if (PZ) add(i - (n - nxy), Wz);
+#pragma unroll
+		for (int q = 0; q < 6; ++q) {
+			const V3<T> t = sum + W[q] * (scale_rn(T(1) / msj[q], Mj[q]) - mi);
+			sum = has[q] && msj[q] != T(0) ? t : sum;
+		}
 		const T pre = (T)(2.0 / MU0) * A[i] / ms;
 		const V3<T> Hi = pre * sum;
 		store3(H, i, n, Hi);
-		if (energy) e += (double)dot(Mi, Hi);
+		if (energy.slot) e += (double)dot(Mi, Hi);
 	}
-	if (energy) block_sum_to(energy, e);
+	if (energy.slot) grid_sum_to_host(energy.slot, energy.host, e);
 }
 
 template <typename T>
@@ -72,13 +77,8 @@ mm_status run_exchange(int nx, int ny, int nz, double dx, double dy, double dz, 
                        double *energy_host, cudaStream_t st)
 {
 	const size_t n = (size_t)nx * ny * nz;
-	double *acc = nullptr;
-	ScalarScratch *sc = nullptr;
-	if (energy_host) {
-		MM_TRY(scalar_scratch(&sc));
-		acc = sc->dev;
-		MM_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), st));
-	}
+	ScalarResult acc;
+	if (energy_host) MM_TRY(scalar_result(&acc));
 	const double wx = 1.0 / (dx * dx), wy = 1.0 / (dy * dy), wz = 1.0 / (dz * dz);
 	const T *ms = (const T *)Ms, *a = (const T *)A, *m = (const T *)M;
 	T *h = (T *)H;
@@ -91,9 +91,8 @@ mm_status run_exchange(int nx, int ny, int nz, double dx, double dy, double dz, 
 #undef MM_EXCH
 	MM_TRY(after_launch("k_exchange"));
 	if (energy_host) {
-		MM_CUDA(cudaMemcpyAsync(sc->host, acc, sizeof(double), cudaMemcpyDeviceToHost, st));
 		MM_CUDA(cudaStreamSynchronize(st));
-		*energy_host = -MU0 / 2.0 * sc->host[0] * dx * dy * dz;
+		*energy_host = -MU0 / 2.0 * *acc.host * dx * dy * dz;
 	}
 	return MM_OK;
 }
@@ -103,7 +102,7 @@ template <typename T>
 __global__ void __launch_bounds__(TPB) k_uniaxial(size_t n, const T *__restrict__ axis,
                                                   const T *__restrict__ k, const T *__restrict__ Ms,
                                                   const T *__restrict__ M, T *__restrict__ H,
-                                                  double *energy)
+                                                  ScalarResult energy)
 {
 	double e = 0.0;
 	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
@@ -117,12 +116,12 @@ __global__ void __launch_bounds__(TPB) k_uniaxial(size_t n, const T *__restrict_
 		const V3<T> s = (T(1) / ms) * load3(M, i, n);
 		const T d = dot(s, a);
 		store3(H, i, n, (T(2) * kk * d / ms / (T)MU0) * a);
-		if (energy) {
+		if (energy.slot) {
 			const V3<T> c = cross(a, s);
 			e += (double)kk * (double)dot(c, c);
 		}
 	}
-	if (energy) block_sum_to(energy, e);
+	if (energy.slot) grid_sum_to_host(energy.slot, energy.host, e);
 }
 
 // ---- cubic anisotropy (anisotropy_cpu.cpp:75-119) ---------------------------------------------
@@ -130,7 +129,7 @@ template <typename T>
 __global__ void __launch_bounds__(TPB) k_cubic(size_t n, const T *__restrict__ axis1,
                                                const T *__restrict__ axis2, const T *__restrict__ k,
                                                const T *__restrict__ Ms, const T *__restrict__ M,
-                                               T *__restrict__ H, double *energy)
+                                               T *__restrict__ H, ScalarResult energy)
 {
 	double e = 0.0;
 	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
@@ -150,9 +149,9 @@ __global__ void __launch_bounds__(TPB) k_cubic(size_t n, const T *__restrict__ a
 		const T a1s = a1 * a1, a2s = a2 * a2, a3s = a3 * a3;
 		const V3<T> h = ((a2s + a3s) * a1) * u1 + ((a1s + a3s) * a2) * u2 + ((a1s + a2s) * a3) * u3;
 		store3(H, i, n, ((T)(-2.0 / MU0) * kk / ms) * h);
-		if (energy) e += (double)kk * (double)(a1s * a2s + a1s * a3s + a2s * a3s);
+		if (energy.slot) e += (double)kk * (double)(a1s * a2s + a1s * a3s + a2s * a3s);
 	}
-	if (energy) block_sum_to(energy, e);
+	if (energy.slot) grid_sum_to_host(energy.slot, energy.host, e);
 }
 
 // ---- LLG right-hand side (mmm/llge/llge_cpu.cpp:25-45) ----------------------------------------
@@ -198,9 +197,9 @@ __global__ void __launch_bounds__(TPB) k_zhangli(int nx, int ny, int nz, double 
 		const V3<T> Mi = load3(M, i, n);
 		auto grad = [&](int c, int dim, size_t stride, double d) -> V3<T> {
 			if (dim <= 1) return v3<T>(0, 0, 0);
-			if (c == 0) return (T)(1.0 / d) * (load3(M, i + stride, n) - Mi);
-			if (c == dim - 1) return (T)(1.0 / d) * (Mi - load3(M, i - stride, n));
-			return (T)(1.0 / (2 * d)) * (load3(M, i + stride, n) - load3(M, i - stride, n));
+			const bool lo = c == 0, hi = c == dim - 1;  // one-sided at the faces (loads before selects, as above)
+			const V3<T> l = load3(M, lo ? i : i - stride, n), r = load3(M, hi ? i : i + stride, n);
+			return (T)(lo || hi ? 1.0 / d : 1.0 / (2 * d)) * (r - l);
 		};
 		const V3<T> gx = grad(x, nx, 1, dx), gy = grad(y, ny, nx, dy), gz = grad(z, nz, nxy, dz);
 		const V3<T> j = load3(J, i, n);
@@ -230,7 +229,7 @@ __global__ void __launch_bounds__(TPB) k_zhangli(int nx, int ny, int nz, double 
 // ---- scaled_abs_max (math/ScaledAbsMax.cpp:33-68) ---------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(TPB) k_scaled_abs_max(size_t n, const T *__restrict__ M,
-                                                        const T *__restrict__ s, double *out)
+                                                        const T *__restrict__ s, ScalarResult out)
 {
 	double best = 0.0;
 	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
@@ -240,7 +239,7 @@ __global__ void __launch_bounds__(TPB) k_scaled_abs_max(size_t n, const T *__res
 		const double mx = M[i], my = M[i + n], mz = M[i + 2 * n];
 		best = fmax(best, (mx * mx + my * my + mz * mz) / (si * si));
 	}
-	block_max_to(out, best);
+	grid_max_to_host(out.slot, out.host, best);
 }
 
 // ---- normalisation (kernels_simple.cu:88-103, the GPU path's semantics) -----------------------
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__(TPB) k_rk_combine(size_t n3, int nk, double h,
 template <typename T>
 __global__ void __launch_bounds__(TPB) k_rk_error_norm2(size_t n3, double eps_abs, double eps_rel,
                                                         const T *__restrict__ y, const T *__restrict__ yerr,
-                                                        double *out)
+                                                        ScalarResult out)
 {
 	double acc = 0.0;
 	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n3;
@@ -308,15 +307,14 @@ __global__ void __launch_bounds__(TPB) k_rk_error_norm2(size_t n3, double eps_ab
 		const double r = fabs((double)yerr[i]) / fabs(d0);
 		acc += r * r;
 	}
-	block_sum_to(out, acc);
+	grid_sum_to_host(out.slot, out.host, acc);
 }
 
-template <typename T>
-mm_status finish_energy(double *acc, ScalarScratch *sc, double *energy_host, cudaStream_t st)
+// Waits for a scalar result and reads it.
+mm_status finish_scalar(const ScalarResult &r, double *out, cudaStream_t st)
 {
-	MM_CUDA(cudaMemcpyAsync(sc->host, acc, sizeof(double), cudaMemcpyDeviceToHost, st));
 	MM_CUDA(cudaStreamSynchronize(st));
-	*energy_host = sc->host[0];
+	*out = *r.host;
 	return MM_OK;
 }
 
@@ -350,13 +348,8 @@ MM_API mm_status mm_uniaxial_anisotropy(int prec, size_t n, const void *axis, co
 	if (bad_prec(prec) || n == 0 || !axis || !k || !Ms || !M || !H)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_uniaxial_anisotropy: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	double *acc = nullptr;
-	ScalarScratch *sc = nullptr;
-	if (energy_host) {
-		MM_TRY(scalar_scratch(&sc));
-		acc = sc->dev;
-		MM_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), st));
-	}
+	ScalarResult acc;
+	if (energy_host) MM_TRY(scalar_result(&acc));
 	if (prec == MM_F64)
 		k_uniaxial<double><<<grid_for(n), TPB, 0, st>>>(n, (const double *)axis, (const double *)k,
 		                                                (const double *)Ms, (const double *)M,
@@ -366,7 +359,7 @@ MM_API mm_status mm_uniaxial_anisotropy(int prec, size_t n, const void *axis, co
 		                                               (const float *)Ms, (const float *)M,
 		                                               (float *)H, acc);
 	MM_TRY(after_launch("k_uniaxial"));
-	if (energy_host) return finish_energy<double>(acc, sc, energy_host, st);
+	if (energy_host) return finish_scalar(acc, energy_host, st);
 	return MM_OK;
 }
 
@@ -377,13 +370,8 @@ MM_API mm_status mm_cubic_anisotropy(int prec, size_t n, const void *axis1, cons
 	if (bad_prec(prec) || n == 0 || !axis1 || !axis2 || !k || !Ms || !M || !H)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_cubic_anisotropy: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	double *acc = nullptr;
-	ScalarScratch *sc = nullptr;
-	if (energy_host) {
-		MM_TRY(scalar_scratch(&sc));
-		acc = sc->dev;
-		MM_CUDA(cudaMemsetAsync(acc, 0, sizeof(double), st));
-	}
+	ScalarResult acc;
+	if (energy_host) MM_TRY(scalar_result(&acc));
 	if (prec == MM_F64)
 		k_cubic<double><<<grid_for(n), TPB, 0, st>>>(n, (const double *)axis1, (const double *)axis2,
 		                                             (const double *)k, (const double *)Ms,
@@ -393,7 +381,7 @@ MM_API mm_status mm_cubic_anisotropy(int prec, size_t n, const void *axis1, cons
 		                                            (const float *)k, (const float *)Ms,
 		                                            (const float *)M, (float *)H, acc);
 	MM_TRY(after_launch("k_cubic"));
-	if (energy_host) return finish_energy<double>(acc, sc, energy_host, st);
+	if (energy_host) return finish_scalar(acc, energy_host, st);
 	return MM_OK;
 }
 
@@ -441,19 +429,18 @@ MM_API mm_status mm_scaled_abs_max(int prec, size_t n, const void *M, const void
 	if (bad_prec(prec) || n == 0 || !M || !scale || !result_host)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_scaled_abs_max: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	ScalarScratch *sc = nullptr;
-	MM_TRY(scalar_scratch(&sc));
-	MM_CUDA(cudaMemsetAsync(sc->dev, 0, sizeof(double), st));
+	ScalarResult sc;
+	MM_TRY(scalar_result(&sc));
 	if (prec == MM_F64)
 		k_scaled_abs_max<double><<<grid_for(n), TPB, 0, st>>>(n, (const double *)M,
-		                                                      (const double *)scale, sc->dev);
+		                                                      (const double *)scale, sc);
 	else
 		k_scaled_abs_max<float><<<grid_for(n), TPB, 0, st>>>(n, (const float *)M,
-		                                                     (const float *)scale, sc->dev);
+		                                                     (const float *)scale, sc);
 	MM_TRY(after_launch("k_scaled_abs_max"));
-	MM_CUDA(cudaMemcpyAsync(sc->host, sc->dev, sizeof(double), cudaMemcpyDeviceToHost, st));
-	MM_CUDA(cudaStreamSynchronize(st));
-	*result_host = sqrt(sc->host[0]);
+	double r = 0.0;
+	MM_TRY(finish_scalar(sc, &r, st));
+	*result_host = sqrt(r);
 	return MM_OK;
 }
 
@@ -463,20 +450,19 @@ MM_API mm_status mm_rk_scaled_error_norm(int prec, size_t n, double eps_abs, dou
 	if (bad_prec(prec) || n == 0 || !y || !y_error || !norm_host)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_rk_scaled_error_norm: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	ScalarScratch *sc = nullptr;
-	MM_TRY(scalar_scratch(&sc));
-	MM_CUDA(cudaMemsetAsync(sc->dev, 0, sizeof(double), st));
+	ScalarResult sc;
+	MM_TRY(scalar_result(&sc));
 	const size_t n3 = 3 * n;
 	if (prec == MM_F64)
 		k_rk_error_norm2<double><<<grid_for(n3), TPB, 0, st>>>(n3, eps_abs, eps_rel, (const double *)y,
-		                                                       (const double *)y_error, sc->dev);
+		                                                       (const double *)y_error, sc);
 	else
 		k_rk_error_norm2<float><<<grid_for(n3), TPB, 0, st>>>(n3, eps_abs, eps_rel, (const float *)y,
-		                                                      (const float *)y_error, sc->dev);
+		                                                      (const float *)y_error, sc);
 	MM_TRY(after_launch("k_rk_error_norm2"));
-	MM_CUDA(cudaMemcpyAsync(sc->host, sc->dev, sizeof(double), cudaMemcpyDeviceToHost, st));
-	MM_CUDA(cudaStreamSynchronize(st));
-	*norm_host = sqrt(sc->host[0] / (double)n3);
+	double r = 0.0;
+	MM_TRY(finish_scalar(sc, &r, st));
+	*norm_host = sqrt(r / (double)n3);
 	return MM_OK;
 }
 
