@@ -19,7 +19,7 @@ struct ConvPlan {
 	int qy = 0, qz = 0;             // py/2 + 1, pz/2 + 1 stored tensor frequencies
 	bool is2d = false;              // nz == 1 && pz == 1
 	bool fast_x = false, fast_y = false, fast_z = false;  // compile-time register-FFT passes (2^k, 3 * 2^k)
-	bool reg_z = false;             // z pass with whole columns in registers (nz <= pz/2, pz small)
+	bool reg_z = false;             // z pass with whole columns in registers (nz <= pz/2, pz up to 32)
 	bool tma_y = false;             // y passes fed by TMA-staged tiles (persistent CTAs)
 	CUtensorMap tm_yf{}, tm_yi{};   // spectrum views of the forward (ny rows) and inverse (py rows) y pass
 	int grid_yf = 0, grid_yi = 0;   // persistent grid sizes of those passes
@@ -36,7 +36,7 @@ struct ConvPlan {
 	const void *xr_ptr = nullptr;         // region map the region tensor map was encoded for
 	CUtensorMap xr_map{};                 // region bytes of the forward pass's rows
 	FftRadices rx{}, ry{}, rz{};
-	void *tw_x = nullptr, *tw_y = nullptr, *tw_z = nullptr;  // cplx<T> twiddle tables
+	void *tw_x = nullptr, *tw_y = nullptr, *tw_z = nullptr;  // cplx<T> twiddle tables (plain, then per pass)
 	void *tensor = nullptr;         // reduced real tensor spectrum, T[6][qz][qy][hx]
 	void *tensor_kx = nullptr;      // the same, kx-major T[hx][qz][qy][6] (made by the first grouped
 	                                // convolution whose fused y+z pass takes this plan)

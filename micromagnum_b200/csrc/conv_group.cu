@@ -881,7 +881,6 @@ mm_status group_create(ConvGroup *g, const ConvGroupMember *m, int count, cudaSt
 
 mm_status conv_group_create(ConvGroup **out, const ConvGroupMember *members, int count, cudaStream_t st)
 {
-	MM_TRY(fft_reg_init());  // this translation unit's tables
 	if (!out || !members || count < 1) return fail(MM_ERR_INVALID_ARGUMENT, "conv group: no members");
 	ConvGroup *g = new ConvGroup();
 	g->prec = members[0].plan ? members[0].plan->prec : MM_F32;

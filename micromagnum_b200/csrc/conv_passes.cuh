@@ -456,6 +456,15 @@ __global__ void __launch_bounds__(TB * (N / ct_radix(N)), 2) k_y_ct(cplx<T> *__r
 
 __device__ const uint8_t g_region0 = 0;
 
+// Spectrum rows of the real rows ra and ra + 1 (row (c nz + z) ny + y has row (c nz + z) py + y); row 0 for
+// one that does not exist.
+__device__ __forceinline__ void spec_rows(int ra, bool va, bool vb, int ny, int py, size_t &sa, size_t &sb)
+{
+	const int plane = (va ? ra : 0) / ny, y = (va ? ra : 0) - plane * ny;
+	sa = (size_t)plane * py + y;
+	sb = !vb ? 0 : y + 1 < ny ? sa + 1 : (size_t)(plane + 1) * py;
+}
+
 // x pass forward: LPB complex lines per CTA (line q packs real rows 2q, 2q+1).
 template <typename T, int N, int LPB, bool SCALE, int R = ct_radix(N), bool H0 = false>
 __device__ __forceinline__ void x_fwd_ct_body(const T *__restrict__ M, const uint8_t *__restrict__ reg,
@@ -495,24 +504,29 @@ __device__ __forceinline__ void x_fwd_ct_body(const T *__restrict__ M, const uin
 	if constexpr (H0) cta_fft_h0<T, N, R, LPB, SI>(sm, twN, line, j0, ld, st);
 	else cta_fft<T, N, R, LPB, false, SI>(sm, twN, line, j0, ld, st);
 	__syncthreads();
-	C *Sa = S + ((size_t)(qa / nyz * nz + qa % nyz / ny) * py + qa % nyz % ny) * lx;
-	C *Sb = S + ((size_t)(qb / nyz * nz + qb % nyz / ny) * py + qb % nyz % ny) * lx;
+	size_t sa, sb;
+	spec_rows(ra, va, vb, ny, py, sa, sb);
+	C *Sa = S + sa * lx, *Sb = S + sb * lx;
 	const T h = T(0.5);
-	for (int k = j0; k < hx; k += TPL) {
+	auto out = [&](int k) {
 		const C zk = sm[SI::at(line, k)], zn = sm[SI::at(line, k == 0 ? 0 : N - k)];
 		if (va) Sa[k] = C{h * (zk.x + zn.x), h * (zk.y - zn.y)};
 		if (vb) Sb[k] = C{h * (zk.y + zn.y), h * (zn.x - zk.x)};
-	}
+	};
+#pragma unroll
+	for (int i = 0; i < R / 2; ++i) out(j0 + i * TPL);  // k < N/2, then the last stored frequency
+	if (j0 == 0) out(N / 2);
 }
 
-template <typename T, int N, int LPB, bool SCALE>
+// H0: at most N/2 samples, the upper half of the inputs is zero padding (not along a periodic axis).
+template <typename T, int N, int LPB, bool SCALE, bool H0>
 __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_fwd_ct(const T *__restrict__ M,
                                                                      const uint8_t *__restrict__ reg,
                                                                      const T *__restrict__ ms_tab,
                                                                      cplx<T> *__restrict__ S, int nx, int ny, int nz,
                                                                      int py, int hx, int lx, const cplx<T> *__restrict__ twN)
 {
-	x_fwd_ct_body<T, N, LPB, SCALE>(M, reg, ms_tab, S, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
+	x_fwd_ct_body<T, N, LPB, SCALE, ct_radix(N), H0>(M, reg, ms_tab, S, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
 }
 
 // x pass inverse: half spectra of rows 2q, 2q+1 -> real rows.
@@ -531,11 +545,12 @@ __device__ __forceinline__ void x_inv_ct_body(const cplx<T> *__restrict__ S, T *
 	const int ra = 2 * (blk * LPB + line), rb = ra + 1;
 	const bool va = ra < rows, vb = rb < rows;
 	const int qa = va ? ra : 0, qb = vb ? rb : 0;
-	const C *Sa = S + ((size_t)(qa / nyz * nz + qa % nyz / ny) * py + qa % nyz % ny) * lx;
-	const C *Sb = S + ((size_t)(qb / nyz * nz + qb % nyz / ny) * py + qb % nyz % ny) * lx;
+	size_t sa, sb;
+	spec_rows(ra, va, vb, ny, py, sa, sb);
+	const C *Sa = S + sa * lx, *Sb = S + sb * lx;
 	T *Ha = H + (size_t)qa * nx, *Hb = H + (size_t)qb * nx;
 	auto ld = [&](int, int f) -> C {
-		const bool mirror = f >= hx;
+		const bool mirror = 2 * f > N;
 		const int ff = mirror ? N - f : f;
 		C A = Sa[ff], B = Sb[ff];
 		if (!vb) B = C{0, 0};
@@ -996,7 +1011,6 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 		const uint8_t *rgb = rga + nx;
 		const int ra = 2 * (t * LPB + line), rb = ra + 1;
 		const bool va = ra < rows, vb = rb < rows;
-		const int qa = va ? ra : 0, qb = vb ? rb : 0;
 		// loads first, selects afterwards (as x_fwd_ct_body); x < N/2 stays inside the stage buffer, and
 		// whatever byte lies there is an index of the 256-entry table
 		auto ld = [&](int, int x) -> C {
@@ -1018,14 +1032,18 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 		};
 		cta_fft_h0<T, N, G::R, LPB, SI>(work, tws, line, j0, ld, st, release);  // x >= nx, N/2 <= x: zero
 		__syncthreads();
-		C *Sa = S + ((size_t)(qa / nyz * nz + qa % nyz / ny) * py + qa % nyz % ny) * lx;
-		C *Sb = S + ((size_t)(qb / nyz * nz + qb % nyz / ny) * py + qb % nyz % ny) * lx;
+		size_t sa, sb;
+		spec_rows(ra, va, vb, ny, py, sa, sb);
+		C *Sa = S + sa * lx, *Sb = S + sb * lx;
 		const T h = T(0.5);
-		for (int kk = j0; kk < hx; kk += TPL) {
+		auto out = [&](int kk) {
 			const C zk = work[SI::at(line, kk)], zn = work[SI::at(line, kk == 0 ? 0 : N - kk)];
 			if (va) Sa[kk] = C{h * (zk.x + zn.x), h * (zk.y - zn.y)};
 			if (vb) Sb[kk] = C{h * (zk.y + zn.y), h * (zn.x - zk.x)};
-		}
+		};
+#pragma unroll
+		for (int i = 0; i < G::R / 2; ++i) out(j0 + i * TPL);  // k < N/2, then the last stored frequency
+		if (j0 == 0) out(N / 2);
 	}
 }
 
@@ -1081,7 +1099,7 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 		const size_t ra = 2 * ((size_t)t * LPB + line);
 		T *Ha = H + ra * nx, *Hb = Ha + nx;
 		auto ld = [&](int, int f) -> C {
-			const bool mirror = f >= hx;
+			const bool mirror = 2 * f > N;
 			const int ff = mirror ? N - f : f;
 			C A = Sa[ff], B = Sb[ff];
 			if (ff == 0 || 2 * ff == N) { A.y = 0; B.y = 0; }
@@ -1160,8 +1178,10 @@ mm_status fs_setup_len()
 	const size_t sx = (size_t)SmRows<N, LPB>::SIZE * sizeof(C), sy = (size_t)SmCols<N, TB>::SIZE * sizeof(C);
 	MM_TRY(set_smem<T>((const void *)k_y2d_ct<T, N, T2>, (size_t)SmCols<N, 3 * T2>::SIZE * sizeof(C)));
 	MM_TRY(set_smem<T>((const void *)k_y2d_ct<T, N, 1>, (size_t)SmCols<N, 3>::SIZE * sizeof(C)));
-	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, false>, sx));
-	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, true>, sx));
+	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, false, false>, sx));
+	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, true, false>, sx));
+	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, false, true>, sx));
+	MM_TRY(set_smem<T>((const void *)k_x_fwd_ct<T, N, LPB, true, true>, sx));
 	MM_TRY(set_smem<T>((const void *)k_x_inv_ct<T, N, LPB>, sx));
 	MM_TRY(set_smem<T>((const void *)k_y_ct<T, N, TB, false>, sy));
 	MM_TRY(set_smem<T>((const void *)k_y_ct<T, N, TB, true>, sy));
@@ -1362,19 +1382,24 @@ void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cuda
 	using C = cplx<T>;
 	constexpr int TPL = N / ct_radix(N);
 	const int lines = (3 * p->ny * p->nz + 1) / 2;
-	auto go = [&](auto lpb) {
+	auto go = [&](auto lpb, auto half) {
 		constexpr int LPB = decltype(lpb)::value;
+		constexpr bool H0 = decltype(half)::value;
 		const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
 		const size_t smem = (size_t)SmRows<N, LPB>::SIZE * sizeof(C);
 		if (ms_tab)
-			k_x_fwd_ct<T, N, LPB, true><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
+			k_x_fwd_ct<T, N, LPB, true, H0><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
 		                                                       p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
 		else
-			k_x_fwd_ct<T, N, LPB, false><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
+			k_x_fwd_ct<T, N, LPB, false, H0><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
 			                                                        p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
 	};
-	if (fs_narrow_x<T, N>(p)) go(std::integral_constant<int, ct_lpb_narrow(N)>());
-	else go(std::integral_constant<int, ct_lpb(N, sizeof(C))>());
+	auto pick = [&](auto half) {
+		if (fs_narrow_x<T, N>(p)) go(std::integral_constant<int, ct_lpb_narrow(N)>(), half);
+		else go(std::integral_constant<int, ct_lpb(N, sizeof(C))>(), half);
+	};
+	if (2 * p->nx <= N) pick(std::true_type());
+	else pick(std::false_type());
 }
 
 template <typename T, int N>
@@ -1469,7 +1494,6 @@ void fs_z(ConvPlan *p, cudaStream_t st)
 template <typename T>
 mm_status fs_setup(ConvPlan *p)
 {
-	MM_TRY(fft_reg_init());
 	// (the staged and register passes skip the zero upper half of a forward transform; an axis without
 	// zero padding, a periodic one of padded length n, takes those that load every input)
 	p->fast_x = fs_len_ok<T>(p->px);

@@ -1,45 +1,82 @@
-// Register-resident FFT building blocks for power-of-two lengths (included by conv.cu only).
+// Register-resident FFT building blocks for lengths 2^k and 3 * 2^k (included by conv_passes.cuh).
 //
-// dft_reg<T, N, INV>: an N-point DFT (N = 1..64) held entirely in one thread's registers,
-// radix-4 decimation in frequency (a radix-2 stage last where 4 does not divide, after one radix-3
-// stage for N = 3 * 2^k <= 48), fully unrolled, output k in register dft_pos<N>(k).  Its twiddles W_64^q = exp(-2 pi i q / 64) live in a __constant__ table that every
-// lane reads at the same compile-time index (a broadcast).
+// dft_reg<T, N, INV>: an N-point DFT (N up to 64, or 3 * 2^k up to 48) held entirely in one thread's
+// registers, radix-4 decimation in frequency (a radix-2 stage last where 4 does not divide, after one
+// radix-3 stage for N = 3 * 2^k), fully unrolled, output k in register dft_pos<N>(k).  Its twiddles are
+// compile-time constants.
 //
-// Longer transforms (N = N1 * N2 <= 4096) use the four-step decomposition within a CTA:
-//   X[f1 + N1 f2] = sum_t W_N2^(t f2) W_N^(t f1) sum_k x[t + N2 k] W_N1^(k f1)
-// i.e. N2 threads each do an N1-point register DFT, multiply by W_N^(t f1), exchange through
-// shared memory once, and finish with N2-point register DFTs.  No index arithmetic depends on
-// runtime values except the tile offsets, so the inner work is straight-line code.
+// Longer transforms are CTA-wide Stockham passes over shared memory (cta_fft below).  No index
+// arithmetic depends on run-time values except the tile offsets, so the inner work is straight-line code.
 #pragma once
 
 #include "fft.cuh"
-#include "mm_common.cuh"
-
-#include <cmath>
 
 namespace mm {
 
-static __constant__ double2 c_w64d[64];
-static __constant__ float2 c_w64f[64];
-
+// cos(2 pi q / 64) and cos(2 pi q / 48) for the first quarter, and the rest by symmetry.  Called with
+// constants after unrolling, so the values are operands in the instruction stream: from __constant__
+// tables they were fetched anew by every SM in every launch, which the short launches waited for.
+__host__ __device__ constexpr double cos_q64(int q)
+{
+	switch (q) {
+	case 0: return 1.0;
+	case 1: return 0.99518472667219688624;
+	case 2: return 0.98078528040323044913;
+	case 3: return 0.95694033573220886494;
+	case 4: return 0.92387953251128675613;
+	case 5: return 0.88192126434835502971;
+	case 6: return 0.83146961230254523708;
+	case 7: return 0.77301045336273696081;
+	case 8: return 0.70710678118654752440;
+	case 9: return 0.63439328416364549822;
+	case 10: return 0.55557023301960222474;
+	case 11: return 0.47139673682599764856;
+	case 12: return 0.38268343236508977173;
+	case 13: return 0.29028467725446236764;
+	case 14: return 0.19509032201612826785;
+	case 15: return 0.09801714032956060199;
+	default: return 0.0;
+	}
+}
+__host__ __device__ constexpr double cos_q48(int q)
+{
+	switch (q) {
+	case 0: return 1.0;
+	case 1: return 0.99144486137381041114;
+	case 2: return 0.96592582628906828675;
+	case 3: return 0.92387953251128675613;
+	case 4: return 0.86602540378443864676;
+	case 5: return 0.79335334029123516458;
+	case 6: return 0.70710678118654752440;
+	case 7: return 0.60876142900872063942;
+	case 8: return 0.5;
+	case 9: return 0.38268343236508977173;
+	case 10: return 0.25881904510252076235;
+	case 11: return 0.13052619222005159155;
+	default: return 0.0;
+	}
+}
+// cos(2 pi q / n) for n = 64 or 48, any q >= 0
+__host__ __device__ constexpr double cos_of(int q, int n)
+{
+	q %= n;
+	if (2 * q > n) q = n - q;
+	const bool neg = 4 * q > n;
+	if (neg) q = n / 2 - q;
+	const double c = n == 64 ? cos_q64(q) : cos_q48(q);
+	return neg ? -c : c;
+}
+// W_n^q = exp(-2 pi i q / n): sin(2 pi q / n) = cos(2 pi (q - n / 4) / n)
 template <typename T>
-__device__ __forceinline__ cplx<T> w64(int q);
-template <>
-__device__ __forceinline__ double2 w64<double>(int q) { return c_w64d[q]; }
-template <>
-__device__ __forceinline__ float2 w64<float>(int q) { return c_w64f[q]; }
-
-// W_48^q for the register transforms of 3 * 2^k points.
-static __constant__ double2 c_w48d[48];
-static __constant__ float2 c_w48f[48];
-
+__device__ __forceinline__ cplx<T> w64(int q)
+{
+	return {(T)cos_of(q, 64), (T)-cos_of(q + 48, 64)};
+}
 template <typename T>
-__device__ __forceinline__ cplx<T> w48(int q);
-template <>
-__device__ __forceinline__ double2 w48<double>(int q) { return c_w48d[q]; }
-template <>
-__device__ __forceinline__ float2 w48<float>(int q) { return c_w48f[q]; }
-
+__device__ __forceinline__ cplx<T> w48(int q)
+{
+	return {(T)cos_of(q, 48), (T)-cos_of(q + 36, 48)};
+}
 
 __host__ __device__ constexpr bool fft_is_pow2(int n) { return (n & (n - 1)) == 0; }
 
@@ -325,28 +362,6 @@ __device__ __forceinline__ void cta_fft_h0(cplx<T> *sm, const cplx<T> *__restric
                                            ST &st, HK hk = HK())
 {
 	cta_fft_pass<T, N, R, LANES, false, SmIdx, LD_SM, 0, true>(sm, twp, line, j0, ld, st, hk);
-}
-
-// Uploads this translation unit's tables to the current device (idempotent).
-static inline mm_status fft_reg_init()
-{
-	double2 d[64];
-	float2 f[64];
-	for (int k = 0; k < 64; ++k) {
-		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / 64.0L;
-		d[k] = double2{(double)cosl(a), (double)sinl(a)};
-		f[k] = float2{(float)cosl(a), (float)sinl(a)};
-	}
-	MM_CUDA(cudaMemcpyToSymbol(c_w64d, d, sizeof(d)));
-	MM_CUDA(cudaMemcpyToSymbol(c_w64f, f, sizeof(f)));
-	for (int k = 0; k < 48; ++k) {
-		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / 48.0L;
-		d[k] = double2{(double)cosl(a), (double)sinl(a)};
-		f[k] = float2{(float)cosl(a), (float)sinl(a)};
-	}
-	MM_CUDA(cudaMemcpyToSymbol(c_w48d, d, 48 * sizeof(double2)));
-	MM_CUDA(cudaMemcpyToSymbol(c_w48f, f, 48 * sizeof(float2)));
-	return MM_OK;
 }
 
 } // namespace mm

@@ -772,18 +772,21 @@ __global__ void __launch_bounds__(ST_CONS + 32, StTmaGeom<T>::MINB)
 		if (op_hd >= 0) opmap[op_hd] = &maps.hd;
 		if (op_hi >= 0) opmap[op_hi] = &maps.hi;
 		if (op_lo >= 0) opmap[op_lo] = &maps.lo;
-		for (int l = 0; l < MAXS; ++l) {
+	}
+	// one thread per stage vector (a warp of its own): these loads do not wait for one another
+#pragma unroll
+	for (int l = 0; l < MAXS; ++l)
+		if (tid == 32 + l) {
 			fb[l] = (T)(st->h * sc.bn[l]);
 			fe[l] = (T)(st->h * sc.ec[l]);
+			if (kop[l] >= 0) {
+				const void *p = ktab->k[l];
+				int at = 0;
+#pragma unroll
+				for (int q = 0; q < MAXS; ++q) at = maps.kptr[q] == p ? q : at;
+				opmap[kop[l]] = &maps.k[at];
+			}
 		}
-		for (int l = 0; l < MAXS; ++l) {
-			if (kop[l] < 0) continue;
-			const void *p = ktab->k[l];
-			opmap[kop[l]] = &maps.k[0];
-			for (int q = 0; q < MAXS; ++q)
-				if (maps.kptr[q] == p) opmap[kop[l]] = &maps.k[q];
-		}
-	}
 	load_ms_table(a, msr);  // ends with __syncthreads
 	const long long nsteps = (long long)tiles_x * tiles_y * nz;
 	const int L0 = (int)(nsteps * blockIdx.x / gridDim.x), L1 = (int)(nsteps * (blockIdx.x + 1) / gridDim.x);
