@@ -466,7 +466,7 @@ __device__ __forceinline__ void spec_rows(int ra, bool va, bool vb, int ny, int 
 }
 
 // x pass forward: LPB complex lines per CTA (line q packs real rows 2q, 2q+1).
-template <typename T, int N, int LPB, bool SCALE, int R = ct_radix(N), bool H0 = false>
+template <typename T, int N, int LPB, bool SCALE, int R = ct_radix(N), bool H0 = false, bool PK = true>
 __device__ __forceinline__ void x_fwd_ct_body(const T *__restrict__ M, const uint8_t *__restrict__ reg,
                                               const T *__restrict__ ms_tab, cplx<T> *__restrict__ S, int nx, int ny,
                                               int nz, int py, int hx, int lx, const cplx<T> *__restrict__ twN, int blk)
@@ -501,8 +501,8 @@ __device__ __forceinline__ void x_fwd_ct_body(const T *__restrict__ M, const uin
 		return C{in && va ? a : T(0), in && vb ? b : T(0)};
 	};
 	auto st = [&](int l, int k, C v) { sm[SI::at(l, k)] = v; };
-	if constexpr (H0) cta_fft_h0<T, N, R, LPB, SI>(sm, twN, line, j0, ld, st);
-	else cta_fft<T, N, R, LPB, false, SI>(sm, twN, line, j0, ld, st);
+	if constexpr (H0) cta_fft_h0<T, N, R, LPB, SI, false, PK>(sm, twN, line, j0, ld, st);
+	else cta_fft<T, N, R, LPB, false, SI, false, PK>(sm, twN, line, j0, ld, st);
 	__syncthreads();
 	size_t sa, sb;
 	spec_rows(ra, va, vb, ny, py, sa, sb);
@@ -526,11 +526,11 @@ __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_fwd_ct(const T *_
                                                                      cplx<T> *__restrict__ S, int nx, int ny, int nz,
                                                                      int py, int hx, int lx, const cplx<T> *__restrict__ twN)
 {
-	x_fwd_ct_body<T, N, LPB, SCALE, ct_radix(N), H0>(M, reg, ms_tab, S, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
+	x_fwd_ct_body<T, N, LPB, SCALE, ct_radix(N), H0, LPB != ct_lpb_narrow(N)>(M, reg, ms_tab, S, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
 }
 
 // x pass inverse: half spectra of rows 2q, 2q+1 -> real rows.
-template <typename T, int N, int LPB, int R = ct_radix(N)>
+template <typename T, int N, int LPB, int R = ct_radix(N), bool PK = true>
 __device__ __forceinline__ void x_inv_ct_body(const cplx<T> *__restrict__ S, T *__restrict__ H, int nx, int ny,
                                               int nz, int py, int hx, int lx, const cplx<T> *__restrict__ twN, int blk)
 {
@@ -564,7 +564,7 @@ __device__ __forceinline__ void x_inv_ct_body(const cplx<T> *__restrict__ S, T *
 			if (vb) Hb[x] = v.y;
 		}
 	};
-	cta_fft<T, N, R, LPB, true, SI>(sm, twN, line, j0, ld, st);
+	cta_fft<T, N, R, LPB, true, SI, false, PK>(sm, twN, line, j0, ld, st);
 }
 
 template <typename T, int N, int LPB>
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_inv_ct(const cplx
                                                                      int nx, int ny, int nz, int py, int hx, int lx,
                                                                      const cplx<T> *__restrict__ twN)
 {
-	x_inv_ct_body<T, N, LPB>(S, H, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
+	x_inv_ct_body<T, N, LPB, ct_radix(N), LPB != ct_lpb_narrow(N)>(S, H, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
 }
 
 // y pass with the tensor multiply for 2-D problems (CTA-Stockham form): a CTA takes TB columns of
@@ -608,7 +608,7 @@ __global__ void __launch_bounds__(3 * TB * (N / ct_radix(N)))
 	{
 		auto ld = [&](int, int y) -> C { return (ok && y < ny) ? col[(size_t)y * lx] : C{0, 0}; };
 		auto st = [&](int l, int k, C v) { sm[SI::at(l, k)] = v; };
-		cta_fft<T, N, R, LANES, false, SI>(sm, twN, line, j0, ld, st);
+		cta_fft<T, N, R, LANES, false, SI, false, TB != 1>(sm, twN, line, j0, ld, st);
 	}
 	__syncthreads();
 	// row c of the symmetric tensor (components xx, xy, xz, yy, yz, zz); xy and yz are odd in ky
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(3 * TB * (N / ct_radix(N)))
 	auto st = [&](int, int y, C v) {
 		if (ok && y < ny) col[(size_t)y * lx] = v;
 	};
-	cta_fft<T, N, R, LANES, true, SI, true>(sm, twN, line, j0, ld, st);
+	cta_fft<T, N, R, LANES, true, SI, true, TB != 1>(sm, twN, line, j0, ld, st);
 }
 
 // z pass with the tensor multiply (CTA-Stockham form): lines (c, b) = c * TB + b hold the z
@@ -759,6 +759,7 @@ __device__ __forceinline__ void z_reg_body(cplx<T> *__restrict__ S, const T *__r
 			const T *t = tens + kzr * 192 + lane;
 			const T nxx = t[0], nxy = t[32], nxz = t[64], nyy = t[96], nyz = t[128], nzz = t[160];
 			const int nk = (kzr == 0 || kzr == H) ? 1 : 2;
+			const C xx{nxx, nxx}, yy{nyy, nyy}, zz{nzz, nzz};
 #pragma unroll
 			for (int rr = 0; rr < 2; ++rr) {
 				if (rr && !two) break;
@@ -766,13 +767,13 @@ __device__ __forceinline__ void z_reg_body(cplx<T> *__restrict__ S, const T *__r
 				for (int q = 0; q < 2; ++q) {
 					if (q && nk < 2) break;
 					const int kz = q ? PZ - kzr : kzr;
-					const T sy = rr ? T(-1) : T(1), sz = q ? T(-1) : T(1);
 					C *e = sm + ((rr * PZ + kz) * 3) * 32 + lane;
 					const C m0 = e[0], m1 = e[32], m2 = e[64];
-					const T xy = sy * nxy, xz = sz * nxz, yz = sy * sz * nyz;
-					e[0] = C{nxx * m0.x + xy * m1.x + xz * m2.x, nxx * m0.y + xy * m1.y + xz * m2.y};
-					e[32] = C{xy * m0.x + nyy * m1.x + yz * m2.x, xy * m0.y + nyy * m1.y + yz * m2.y};
-					e[64] = C{xz * m0.x + yz * m1.x + nzz * m2.x, xz * m0.y + yz * m1.y + nzz * m2.y};
+					const T sxy = rr ? -nxy : nxy, sxz = q ? -nxz : nxz, syz = rr != q ? -nyz : nyz;
+					const C xy{sxy, sxy}, xz{sxz, sxz}, yz{syz, syz};
+					e[0] = cfma2(xz, m2, cfma2(xy, m1, cscale2(xx, m0)));
+					e[32] = cfma2(yz, m2, cfma2(yy, m1, cscale2(xy, m0)));
+					e[64] = cfma2(zz, m2, cfma2(yz, m1, cscale2(xz, m0)));
 				}
 			}
 		}

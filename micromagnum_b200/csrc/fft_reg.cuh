@@ -114,7 +114,7 @@ __device__ __forceinline__ cplx<T> mul_w64(cplx<T> v, int q)
 // SPAN0 and SPAN0/2 (and leaves its outputs where they would), so a value passes one twiddle
 // multiplication where two radix-2 stages have two (8 instead of 10 in a 16-point transform, and the
 // smaller rounding error); SPAN0 = N/2 is the full transform.
-template <typename T, int N, bool INV, int SPAN0>
+template <typename T, int N, bool INV, int SPAN0, bool PK = true>
 __device__ __forceinline__ void dif_stages(cplx<T> (&v)[N])
 {
 	using C = cplx<T>;
@@ -125,28 +125,28 @@ __device__ __forceinline__ void dif_stages(cplx<T> (&v)[N])
 #pragma unroll
 			for (int j = 0; j < Q; ++j) {
 				const C x0 = v[b + j], x1 = v[b + j + Q], x2 = v[b + j + 2 * Q], x3 = v[b + j + 3 * Q];
-				const C s0 = cadd(x0, x2), d0 = csub(x0, x2), s1 = cadd(x1, x3), d1 = mul_mi<INV>(csub(x1, x3));
+				const C s0 = cadd_pk<PK>(x0, x2), d0 = csub_pk<PK>(x0, x2), s1 = cadd_pk<PK>(x1, x3), d1 = csub_pk<PK>(x1, x3);
 				const int q = j * (64 / (4 * Q));  // W_4Q^j = W_64^q
-				v[b + j] = cadd(s0, s1);
-				v[b + j + Q] = mul_w64<T, INV>(csub(s0, s1), 2 * q);
-				v[b + j + 2 * Q] = mul_w64<T, INV>(cadd(d0, d1), q);
-				v[b + j + 3 * Q] = mul_w64<T, INV>(csub(d0, d1), 3 * q);
+				v[b + j] = cadd_pk<PK>(s0, s1);
+				v[b + j + Q] = mul_w64<T, INV>(csub_pk<PK>(s0, s1), 2 * q);
+				v[b + j + 2 * Q] = mul_w64<T, INV>(cadd_mi<INV>(d0, d1), q);
+				v[b + j + 3 * Q] = mul_w64<T, INV>(csub_mi<INV>(d0, d1), 3 * q);
 			}
 		}
-		if constexpr (Q >= 2) dif_stages<T, N, INV, Q / 2>(v);
+		if constexpr (Q >= 2) dif_stages<T, N, INV, Q / 2, PK>(v);
 	} else if constexpr (SPAN0 == 1) {
 #pragma unroll
 		for (int b = 0; b < N; b += 2) {
 			const C a = v[b], c = v[b + 1];
-			v[b] = cadd(a, c);
-			v[b + 1] = csub(a, c);
+			v[b] = cadd_pk<PK>(a, c);
+			v[b + 1] = csub_pk<PK>(a, c);
 		}
 	}
 }
 
 // N = 3 M points (M a power of two, N <= 48): one radix-3 stage over the inputs M apart, the
 // twiddles W_N^(r j), then three M-point transforms in place.  Outputs at dft_pos<N>.
-template <typename T, int N, bool INV>
+template <typename T, int N, bool INV, bool PK = true>
 __device__ __forceinline__ void dft_reg3(cplx<T> (&v)[N])
 {
 	using C = cplx<T>;
@@ -157,10 +157,10 @@ __device__ __forceinline__ void dft_reg3(cplx<T> (&v)[N])
 #pragma unroll
 	for (int j = 0; j < M; ++j) {
 		const C a = v[j], b = v[j + M], c = v[j + 2 * M];
-		const C s = cadd(b, c), d = csub(b, c);
+		const C s = cadd_pk<PK>(b, c), d = csub_pk<PK>(b, c);
 		const C t = C{a.x - T(0.5) * s.x, a.y - T(0.5) * s.y};
 		const C r = mul_mi<INV>(C{s60 * d.x, s60 * d.y});
-		y[0][j] = cadd(a, s);
+		y[0][j] = cadd_pk<PK>(a, s);
 		C y1 = cadd(t, r), y2 = csub(t, r);
 		if (j > 0) {
 			C w1 = w48<T>(j * (48 / N)), w2 = w48<T>(2 * j * (48 / N));
@@ -176,41 +176,41 @@ __device__ __forceinline__ void dft_reg3(cplx<T> (&v)[N])
 	}
 #pragma unroll
 	for (int r = 0; r < 3; ++r) {
-		if constexpr (M > 1) dif_stages<T, M, INV, M / 2>(y[r]);
+		if constexpr (M > 1) dif_stages<T, M, INV, M / 2, PK>(y[r]);
 #pragma unroll
 		for (int j = 0; j < M; ++j) v[r * M + j] = y[r][j];
 	}
 }
 
-template <typename T, int N, bool INV>
+template <typename T, int N, bool INV, bool PK = true>
 __device__ __forceinline__ void dft_reg(cplx<T> (&v)[N])
 {
-	if constexpr (fft_is_pow2(N)) dif_stages<T, N, INV, N / 2>(v);
-	else dft_reg3<T, N, INV>(v);
+	if constexpr (fft_is_pow2(N)) dif_stages<T, N, INV, N / 2, PK>(v);
+	else dft_reg3<T, N, INV, PK>(v);
 }
 
 // Forward DFT of a column whose upper half v[N/2..N) is zero padding: the first stage's butterflies
 // have two inputs.  Output at dft_pos<N>, like dft_reg.
-template <typename T, int N>
+template <typename T, int N, bool PK = true>
 __device__ __forceinline__ void dft_reg_halfzero(cplx<T> (&v)[N])
 {
 	using C = cplx<T>;
 	if constexpr (!fft_is_pow2(N)) {
 #pragma unroll
 		for (int j = N / 2; j < N; ++j) v[j] = C{T(0), T(0)};
-		dft_reg3<T, N, false>(v);
+		dft_reg3<T, N, false, PK>(v);
 	} else if constexpr (N >= 4) {
 		constexpr int Q = N / 4;
 #pragma unroll
 		for (int j = 0; j < Q; ++j) {
-			const C x0 = v[j], x1 = v[j + Q], r1 = mul_mi<false>(x1);
+			const C x0 = v[j], x1 = v[j + Q];
 			const int q = j * (64 / N);
-			v[j] = cadd(x0, x1);
-			v[j + Q] = mul_w64<T, false>(csub(x0, x1), 2 * q);
-			v[j + 2 * Q] = mul_w64<T, false>(cadd(x0, r1), q);
-			v[j + 3 * Q] = mul_w64<T, false>(csub(x0, r1), 3 * q);
+			v[j] = cadd_pk<PK>(x0, x1);
+			v[j + Q] = mul_w64<T, false>(csub_pk<PK>(x0, x1), 2 * q);
+			v[j + 2 * Q] = mul_w64<T, false>(cadd_mi<false>(x0, x1), q);
+			v[j + 3 * Q] = mul_w64<T, false>(csub_mi<false>(x0, x1), 3 * q);
 		}
-		if constexpr (Q >= 2) dif_stages<T, N, false, Q / 2>(v);
+		if constexpr (Q >= 2) dif_stages<T, N, false, Q / 2, PK>(v);
 	} else if constexpr (N == 2) {
 		v[1] = v[0];
 	}
@@ -290,7 +290,7 @@ struct NoHook {
 
 // H0: the inputs at k >= N/2 are zero (a forward transform of zero-padded data), so pass 0 loads
 // only the lower half of each butterfly's inputs and runs the half-zero register DFT.
-template <typename T, int N, int R, int LANES, bool INV, class SmIdx, bool LD_SM, int p, bool H0, class LD,
+template <typename T, int N, int R, int LANES, bool INV, class SmIdx, bool LD_SM, int p, bool H0, bool PK, class LD,
           class ST, class HK = NoHook>
 __device__ __forceinline__ void cta_fft_pass(cplx<T> *sm, const cplx<T> *__restrict__ twp, int line, int j0,
                                              LD &ld, ST &st, HK hk = HK())
@@ -330,8 +330,8 @@ __device__ __forceinline__ void cta_fft_pass(cplx<T> *sm, const cplx<T> *__restr
 				v[u][q] = cmul(v[u][q], w);
 			}
 		}
-		if constexpr (HALF) dft_reg_halfzero<T, Rp>(v[u]);
-		else dft_reg<T, Rp, INV>(v[u]);
+		if constexpr (HALF) dft_reg_halfzero<T, Rp, PK>(v[u]);
+		else dft_reg<T, Rp, INV, PK>(v[u]);
 		const int base = (j / Ns) * Ns * Rp + jm;
 #pragma unroll
 		for (int k = 0; k < Rp; ++k) {
@@ -342,26 +342,26 @@ __device__ __forceinline__ void cta_fft_pass(cplx<T> *sm, const cplx<T> *__restr
 	}
 	if constexpr (p == 0) hk();
 	if constexpr (p + 1 < P)
-		cta_fft_pass<T, N, R, LANES, INV, SmIdx, LD_SM, p + 1, false>(sm, twp, line, j0, ld, st, hk);
+		cta_fft_pass<T, N, R, LANES, INV, SmIdx, LD_SM, p + 1, false, PK>(sm, twp, line, j0, ld, st, hk);
 }
 
 // LD_SM: the loader reads the same shared memory the passes write (adds a barrier after pass 0's
 // reads).
-template <typename T, int N, int R, int LANES, bool INV, class SmIdx, bool LD_SM = false, class LD, class ST,
-          class HK = NoHook>
+template <typename T, int N, int R, int LANES, bool INV, class SmIdx, bool LD_SM = false, bool PK = true, class LD,
+          class ST, class HK = NoHook>
 __device__ __forceinline__ void cta_fft(cplx<T> *sm, const cplx<T> *__restrict__ twp, int line, int j0, LD &ld,
                                         ST &st, HK hk = HK())
 {
-	cta_fft_pass<T, N, R, LANES, INV, SmIdx, LD_SM, 0, false>(sm, twp, line, j0, ld, st, hk);
+	cta_fft_pass<T, N, R, LANES, INV, SmIdx, LD_SM, 0, false, PK>(sm, twp, line, j0, ld, st, hk);
 }
 
 // Forward transform whose inputs at k >= N/2 are zero (ld is not called for them).
-template <typename T, int N, int R, int LANES, class SmIdx, bool LD_SM = false, class LD, class ST,
-          class HK = NoHook>
+template <typename T, int N, int R, int LANES, class SmIdx, bool LD_SM = false, bool PK = true, class LD,
+          class ST, class HK = NoHook>
 __device__ __forceinline__ void cta_fft_h0(cplx<T> *sm, const cplx<T> *__restrict__ twp, int line, int j0, LD &ld,
                                            ST &st, HK hk = HK())
 {
-	cta_fft_pass<T, N, R, LANES, false, SmIdx, LD_SM, 0, true>(sm, twp, line, j0, ld, st, hk);
+	cta_fft_pass<T, N, R, LANES, false, SmIdx, LD_SM, 0, true, PK>(sm, twp, line, j0, ld, st, hk);
 }
 
 } // namespace mm
