@@ -21,13 +21,6 @@ FftRadices fft_factor(int n)
 	return f;
 }
 
-// conv_f64.cu, conv_f32.cu
-mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
-mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st);
-int conv_fit_length_f64(int n, int e, bool z);
-mm_status conv_setup_f32(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
-mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st);
-int conv_fit_length_f32(int n, int e, bool z);
 
 size_t ConvPlan::spec_bytes() const
 {

@@ -80,8 +80,9 @@ struct ConvGroupMember {
 	const void *M[4];
 	void *H[2];
 	const uint8_t *reg;
-	const void *ms_tab;  // 256 entries (reg NULL: only entry 0 is read, for every cell)
+	const void *ms_tab;  // 256 entries
 	const int *flags;    // device run flags, NULL: always run
+	const void *ms_uniform;  // the one entry that scales every cell (inputs zero where Ms is zero); NULL: by region
 };
 mm_status conv_group_create(ConvGroup **out, const ConvGroupMember *members, int count, cudaStream_t st);
 mm_status conv_group_execute(ConvGroup *g, int input, int gate, cudaStream_t st, int output = 0);
@@ -92,5 +93,15 @@ void conv_group_destroy(ConvGroup *g);
 int conv_group_fused(int prec, int py, int pz, int nz);
 
 FftRadices fft_factor(int n);
+
+// conv_f64.cu, conv_f32.cu (flags, gate: a batch member's run flags, see ConvGroupMember)
+mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
+mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st,
+                       const int *flags = nullptr, int gate = 0);
+int conv_fit_length_f64(int n, int e, bool z);
+mm_status conv_setup_f32(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
+mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st,
+                       const int *flags = nullptr, int gate = 0);
+int conv_fit_length_f32(int n, int e, bool z);
 
 } // namespace mm

@@ -5,9 +5,9 @@ namespace mm {
 
 mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st) { return plan_setup<double>(p, N, octant, st); }
 
-mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st)
+mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st, const int *flags, int gate)
 {
-	return execute<double>(p, M, reg, ms_tab, H, st);
+	return execute<double>(p, M, reg, ms_tab, H, st, Gate{flags, gate});
 }
 
 int conv_fit_length_f64(int n, int e, bool z) { return fit_length<double>(n, e, z); }

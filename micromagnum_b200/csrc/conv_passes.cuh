@@ -39,6 +39,14 @@
 namespace mm {
 namespace {
 
+// Run flags of a batch member whose convolution runs as passes of its own: flags[0] == 0 skips it, and with
+// gate != 0 so does flags[gate] == 0.
+struct Gate {
+	const int *flags = nullptr;
+	int gate = 0;
+	__device__ __forceinline__ bool skip() const { return flags && (!flags[0] || (gate && !flags[gate])); }
+};
+
 constexpr int NT = 256;                 // threads per CTA for all passes
 constexpr size_t SMEM_TARGET = 100 * 1024;
 
@@ -449,8 +457,9 @@ __device__ __forceinline__ void y_ct_body(cplx<T> *__restrict__ S, int n_in, int
 
 template <typename T, int N, int TB, bool INV>
 __global__ void __launch_bounds__(TB * (N / ct_radix(N)), 2) k_y_ct(cplx<T> *__restrict__ S, int n_in, int n_out, int nz,
-                                                                 int hx, int lx, const cplx<T> *__restrict__ twN)
+                                                                 int hx, int lx, const cplx<T> *__restrict__ twN, Gate gate)
 {
+	if (gate.skip()) return;
 	y_ct_body<T, N, TB, INV>(S, n_in, n_out, hx, lx, twN, blockIdx.x, blockIdx.z * nz + blockIdx.y);
 }
 
@@ -524,8 +533,9 @@ __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_fwd_ct(const T *_
                                                                      const uint8_t *__restrict__ reg,
                                                                      const T *__restrict__ ms_tab,
                                                                      cplx<T> *__restrict__ S, int nx, int ny, int nz,
-                                                                     int py, int hx, int lx, const cplx<T> *__restrict__ twN)
+                                                                     int py, int hx, int lx, const cplx<T> *__restrict__ twN, Gate gate)
 {
+	if (gate.skip()) return;
 	x_fwd_ct_body<T, N, LPB, SCALE, ct_radix(N), H0, LPB != ct_lpb_narrow(N)>(M, reg, ms_tab, S, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
 }
 
@@ -570,8 +580,9 @@ __device__ __forceinline__ void x_inv_ct_body(const cplx<T> *__restrict__ S, T *
 template <typename T, int N, int LPB>
 __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_inv_ct(const cplx<T> *__restrict__ S, T *__restrict__ H,
                                                                      int nx, int ny, int nz, int py, int hx, int lx,
-                                                                     const cplx<T> *__restrict__ twN)
+                                                                     const cplx<T> *__restrict__ twN, Gate gate)
 {
+	if (gate.skip()) return;
 	x_inv_ct_body<T, N, LPB, ct_radix(N), LPB != ct_lpb_narrow(N)>(S, H, nx, ny, nz, py, hx, lx, twN, blockIdx.x);
 }
 
@@ -791,17 +802,18 @@ __device__ __forceinline__ void z_reg_body(cplx<T> *__restrict__ S, const T *__r
 
 template <typename T, int PZ>
 __global__ void __launch_bounds__(ZR_THREADS, 2) k_z_reg(cplx<T> *__restrict__ S, const T *__restrict__ Nt, int nz,
-                                                        int py, int hx, int lx, int qy, int qz)
+                                                        int py, int hx, int lx, int qy, int qz, Gate gate)
 {
+	if (gate.skip()) return;
 	z_reg_body<T, PZ>(S, Nt, nz, py, hx, lx, qy, qz, blockIdx.x, blockIdx.y);
 }
 
 template <typename T, int PZ>
-void fs_z_reg(ConvPlan *p, cudaStream_t st)
+void fs_z_reg(ConvPlan *p, cudaStream_t st, Gate gate)
 {
 	const dim3 grid((p->hx + 31) / 32, p->qy);
 	k_z_reg<T, PZ><<<grid, ZR_THREADS, zr_smem<T>(PZ), st>>>(
-	    (cplx<T> *)p->spec, (const T *)p->tensor, p->nz, p->py, p->hx, p->lx, p->qy, p->qz);
+	    (cplx<T> *)p->spec, (const T *)p->tensor, p->nz, p->py, p->hx, p->lx, p->qy, p->qz, gate);
 }
 
 // ---- y pass through TMA-staged tiles -------------------------------------------------------------
@@ -839,8 +851,9 @@ __host__ __device__ constexpr int y_tma_tb(int n, int csize)
 template <typename T, int N, int TB, bool INV>
 __global__ void __launch_bounds__(TB * (N / ct_radix(N)), 2)
     k_y_tma(const __grid_constant__ CUtensorMap tmap, cplx<T> *__restrict__ S, int n_out, int hx, int lx,
-            int tiles_x, int ntiles, const cplx<T> *__restrict__ twN, int *err)
+            int tiles_x, int ntiles, const cplx<T> *__restrict__ twN, int *err, Gate gate)
 {
+	if (gate.skip()) return;
 	using C = cplx<T>;
 	using G = YTmaGeom<N, TB, INV, C>;
 	constexpr int R = ct_radix(N);
@@ -957,8 +970,9 @@ template <typename T, int N, bool SCALE>
 __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cplx<T>>::MINB_F)
     k_x_fwd_tma(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap rmap,
                 const T *__restrict__ ms_tab, cplx<T> *__restrict__ S, int nx, int ny, int nz, int py, int hx,
-                int lx, int ntiles, const cplx<T> *__restrict__ twN, int *err)
+                int lx, int ntiles, const cplx<T> *__restrict__ twN, int *err, Gate gate)
 {
+	if (gate.skip()) return;
 	using C = cplx<T>;
 	using G = XTmaGeom<N, C>;
 	constexpr int LPB = G::LPB, TPL = N / G::R, STG = G::STG_F;
@@ -1053,8 +1067,9 @@ __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cpl
 template <typename T, int N>
 __global__ void __launch_bounds__(XTmaGeom<N, cplx<T>>::THREADS, XTmaGeom<N, cplx<T>>::MINB_I)
     k_x_inv_tma(const __grid_constant__ CUtensorMap tmap, T *__restrict__ H, int nx, int ny, int hx, int lx,
-                int ntiles, const cplx<T> *__restrict__ twN, int *err)
+                int ntiles, const cplx<T> *__restrict__ twN, int *err, Gate gate)
 {
+	if (gate.skip()) return;
 	using C = cplx<T>;
 	using G = XTmaGeom<N, C>;
 	constexpr int LPB = G::LPB, TPL = N / G::R, STG = G::STG_I;
@@ -1238,7 +1253,7 @@ mm_status fs_setup_y_tma(ConvPlan *p)
 }
 
 template <typename T, int N, bool INV>
-void fs_y_tma(ConvPlan *p, cudaStream_t st)
+void fs_y_tma(ConvPlan *p, cudaStream_t st, Gate gate)
 {
 	using C = cplx<T>;
 	constexpr int TB = y_tma_tb(N, sizeof(C)), THREADS = TB * (N / ct_radix(N));
@@ -1247,7 +1262,7 @@ void fs_y_tma(ConvPlan *p, cudaStream_t st)
 	const int grid = std::min(ntiles, INV ? p->grid_yi : p->grid_yf);
 	k_y_tma<T, N, TB, INV><<<grid, THREADS, G::SMEM_TW, st>>>(INV ? p->tm_yi : p->tm_yf, (C *)p->spec,
 	                                                       INV ? p->ny : N, p->hx, p->lx, tiles_x, ntiles,
-	                                                       tw_of((const C *)p->tw_y, N, ct_radix(N)), p->err);
+	                                                       tw_of((const C *)p->tw_y, N, ct_radix(N)), p->err, gate);
 }
 
 // TMA-staged x passes.  The inverse pass's tensor map (over the spectrum) is fixed; the forward
@@ -1340,7 +1355,7 @@ const CUtensorMap *x_fwd_map(ConvPlan *p, const T *M, int lpb)
 }
 
 template <typename T, int N>
-bool fs_x_fwd_tma(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cudaStream_t st)
+bool fs_x_fwd_tma(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cudaStream_t st, Gate gate)
 {
 	using C = cplx<T>;
 	using G = XTmaGeom<N, C>;
@@ -1358,27 +1373,27 @@ bool fs_x_fwd_tma(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	if (ms_tab)
 		k_x_fwd_tma<T, N, true><<<grid, G::THREADS, G::SMEM_F, st>>>(*map, *rmap, ms_tab, (C *)p->spec, p->nx, p->ny,
 		                                                            p->nz, p->py, p->hx, p->lx, ntiles,
-		                                                            tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err);
+		                                                            tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err, gate);
 	else
 		k_x_fwd_tma<T, N, false><<<grid, G::THREADS, G::SMEM_F, st>>>(*map, *rmap, ms_tab, (C *)p->spec, p->nx, p->ny,
 		                                                             p->nz, p->py, p->hx, p->lx, ntiles,
-		                                                             tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err);
+		                                                             tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err, gate);
 	return true;
 }
 
 template <typename T, int N>
-void fs_x_inv_tma(ConvPlan *p, T *H, cudaStream_t st)
+void fs_x_inv_tma(ConvPlan *p, T *H, cudaStream_t st, Gate gate)
 {
 	using C = cplx<T>;
 	using G = XTmaGeom<N, C>;
 	const int ntiles = 3 * p->ny * p->nz / (2 * G::LPB);
 	const int grid = std::min(ntiles, p->grid_xi);
 	k_x_inv_tma<T, N><<<grid, G::THREADS, G::SMEM_I, st>>>(p->tm_xi, H, p->nx, p->ny, p->hx, p->lx, ntiles,
-	                                                     tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err);
+	                                                     tw_of((const C *)p->tw_x, N, ct_radix(N)), p->err, gate);
 }
 
 template <typename T, int N>
-void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cudaStream_t st)
+void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cudaStream_t st, Gate gate)
 {
 	using C = cplx<T>;
 	constexpr int TPL = N / ct_radix(N);
@@ -1390,10 +1405,10 @@ void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cuda
 		const size_t smem = (size_t)SmRows<N, LPB>::SIZE * sizeof(C);
 		if (ms_tab)
 			k_x_fwd_ct<T, N, LPB, true, H0><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
-		                                                       p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+		                                                       p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)), gate);
 		else
 			k_x_fwd_ct<T, N, LPB, false, H0><<<grid, block, smem, st>>>(M, reg, ms_tab, (C *)p->spec, p->nx, p->ny, p->nz,
-			                                                        p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+			                                                        p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)), gate);
 	};
 	auto pick = [&](auto half) {
 		if (fs_narrow_x<T, N>(p)) go(std::integral_constant<int, ct_lpb_narrow(N)>(), half);
@@ -1404,7 +1419,7 @@ void fs_x_fwd(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, cuda
 }
 
 template <typename T, int N>
-void fs_x_inv(ConvPlan *p, T *H, cudaStream_t st)
+void fs_x_inv(ConvPlan *p, T *H, cudaStream_t st, Gate gate)
 {
 	using C = cplx<T>;
 	constexpr int TPL = N / ct_radix(N);
@@ -1413,14 +1428,14 @@ void fs_x_inv(ConvPlan *p, T *H, cudaStream_t st)
 		constexpr int LPB = decltype(lpb)::value;
 		const dim3 grid((lines + LPB - 1) / LPB), block(LPB * TPL);
 		k_x_inv_ct<T, N, LPB><<<grid, block, (size_t)SmRows<N, LPB>::SIZE * sizeof(C), st>>>(
-		    (const C *)p->spec, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)));
+		    (const C *)p->spec, H, p->nx, p->ny, p->nz, p->py, p->hx, p->lx, tw_of((const C *)p->tw_x, N, ct_radix(N)), gate);
 	};
 	if (fs_narrow_x<T, N>(p)) go(std::integral_constant<int, ct_lpb_narrow(N)>());
 	else go(std::integral_constant<int, ct_lpb(N, sizeof(C))>());
 }
 
 template <typename T, int N, bool INV>
-void fs_y(ConvPlan *p, cudaStream_t st)
+void fs_y(ConvPlan *p, cudaStream_t st, Gate gate)
 {
 	using C = cplx<T>;
 	constexpr int TPL = N / ct_radix(N);
@@ -1429,7 +1444,7 @@ void fs_y(ConvPlan *p, cudaStream_t st)
 		const dim3 grid((p->hx + TB - 1) / TB, p->nz, 3), block(TB * TPL);
 		k_y_ct<T, N, TB, INV><<<grid, block, (size_t)SmCols<N, TB>::SIZE * sizeof(C), st>>>(
 		    (C *)p->spec, INV ? N : p->ny, INV ? p->ny : N, p->nz, p->hx, p->lx,
-		    tw_of((const C *)p->tw_y, N, ct_radix(N)));
+		    tw_of((const C *)p->tw_y, N, ct_radix(N)), gate);
 	};
 	if (fs_narrow_y<T, N>(p)) go(std::integral_constant<int, ct_tb_narrow(N, sizeof(C))>());
 	else go(std::integral_constant<int, ct_tb(N, sizeof(C))>());
@@ -1659,7 +1674,7 @@ mm_status plan_setup(ConvPlan *p, const double *N, bool octant, cudaStream_t st)
 }
 
 template <typename T>
-mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, T *H, cudaStream_t st)
+mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, T *H, cudaStream_t st, Gate gate = Gate())
 {
 	using C = cplx<T>;
 	C *S = (C *)p->spec;
@@ -1671,16 +1686,16 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	const double half = 3.0 * p->hx * p->ny * p->nz * c;      // x-transformed rows y < ny, z < nz
 	const double ypad = 3.0 * p->hx * p->py * p->nz * c;      // y-transformed, z < nz
 	const double tens = 6.0 * p->hx * p->qy * p->qz * s;
-	ProfToken tk = prof_begin(st);
+	ProfToken tk = gate.flags ? ProfToken() : prof_begin(st);
 	bool staged = false;
 	if (p->tma_xf) {
-#define MM_XTF(N) staged = fs_x_fwd_tma<T, N>(p, M, reg, ms_tab, st)
+#define MM_XTF(N) staged = fs_x_fwd_tma<T, N>(p, M, reg, ms_tab, st, gate)
 		MM_FS_SWITCH3(p->px, MM_XTF);
 #undef MM_XTF
 	}
 	if (staged) {
 	} else if (p->fast_x) {
-#define MM_XF(N) fs_x_fwd<T, N>(p, M, reg, ms_tab, st)
+#define MM_XF(N) fs_x_fwd<T, N>(p, M, reg, ms_tab, st, gate)
 		MM_FS_SWITCH3(p->px, MM_XF);
 #undef MM_XF
 	} else if (ms_tab)
@@ -1694,7 +1709,7 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 	prof_end(tk, xf_name, 3 * n * s + (reg ? n : 0.0) + half, st);
 	if (p->is2d) {
 		const int gy = (p->hx + p->tb_y - 1) / p->tb_y;
-		tk = prof_begin(st);
+		tk = gate.flags ? ProfToken() : prof_begin(st);
 		if (p->fast_y) {
 #define MM_Y2(N) fs_y2d<T, N>(p, st)
 			MM_FS_SWITCH3(p->py, MM_Y2);
@@ -1707,13 +1722,13 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 		prof_end(tk, y2_name, 2 * half + tens, st);
 	} else {
 		dim3 gy((p->hx + p->tb_y - 1) / p->tb_y, p->nz, 3);
-		tk = prof_begin(st);
+		tk = gate.flags ? ProfToken() : prof_begin(st);
 		if (p->tma_y) {
-#define MM_YTF(N) fs_y_tma<T, N, false>(p, st)
+#define MM_YTF(N) fs_y_tma<T, N, false>(p, st, gate)
 			MM_FS_SWITCH3(p->py, MM_YTF);
 #undef MM_YTF
 		} else if (p->fast_y) {
-#define MM_YF(N) fs_y<T, N, false>(p, st)
+#define MM_YF(N) fs_y<T, N, false>(p, st, gate)
 			MM_FS_SWITCH3(p->py, MM_YF);
 #undef MM_YF
 		} else
@@ -1723,17 +1738,17 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 		MM_TRY(after_launch(yf_name));
 		prof_end(tk, yf_name, half + ypad, st);
 		dim3 gz((p->hx + p->tb_z - 1) / p->tb_z, p->py, 1);
-		tk = prof_begin(st);
+		tk = gate.flags ? ProfToken() : prof_begin(st);
 		if (p->reg_z) {
 			switch (p->pz) {
-			case 2: fs_z_reg<T, 2>(p, st); break;
-			case 6: fs_z_reg<T, 6>(p, st); break;
-			case 12: fs_z_reg<T, 12>(p, st); break;
-			case 24: fs_z_reg<T, 24>(p, st); break;
-			case 4: fs_z_reg<T, 4>(p, st); break;
-			case 8: fs_z_reg<T, 8>(p, st); break;
-			case 16: fs_z_reg<T, 16>(p, st); break;
-			case 32: if constexpr (sizeof(T) == 4) { fs_z_reg<T, 32>(p, st); } break;
+			case 2: fs_z_reg<T, 2>(p, st, gate); break;
+			case 6: fs_z_reg<T, 6>(p, st, gate); break;
+			case 12: fs_z_reg<T, 12>(p, st, gate); break;
+			case 24: fs_z_reg<T, 24>(p, st, gate); break;
+			case 4: fs_z_reg<T, 4>(p, st, gate); break;
+			case 8: fs_z_reg<T, 8>(p, st, gate); break;
+			case 16: fs_z_reg<T, 16>(p, st, gate); break;
+			case 32: if constexpr (sizeof(T) == 4) { fs_z_reg<T, 32>(p, st, gate); } break;
 			}
 		} else if (p->fast_z) {
 			switch (p->pz) {
@@ -1750,13 +1765,13 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 		const char *z_name = p->reg_z ? "k_z_reg" : p->fast_z ? "k_z_ct" : "k_z_mul";
 		MM_TRY(after_launch(z_name));
 		prof_end(tk, z_name, 2 * ypad + tens, st);
-		tk = prof_begin(st);
+		tk = gate.flags ? ProfToken() : prof_begin(st);
 		if (p->tma_y) {
-#define MM_YTI(N) fs_y_tma<T, N, true>(p, st)
+#define MM_YTI(N) fs_y_tma<T, N, true>(p, st, gate)
 			MM_FS_SWITCH3(p->py, MM_YTI);
 #undef MM_YTI
 		} else if (p->fast_y) {
-#define MM_YI(N) fs_y<T, N, true>(p, st)
+#define MM_YI(N) fs_y<T, N, true>(p, st, gate)
 			MM_FS_SWITCH3(p->py, MM_YI);
 #undef MM_YI
 		} else
@@ -1766,13 +1781,13 @@ mm_status execute(ConvPlan *p, const T *M, const uint8_t *reg, const T *ms_tab, 
 		MM_TRY(after_launch(yi_name));
 		prof_end(tk, yi_name, half + ypad, st);
 	}
-	tk = prof_begin(st);
+	tk = gate.flags ? ProfToken() : prof_begin(st);
 	if (p->tma_xi) {
-#define MM_XTI(N) fs_x_inv_tma<T, N>(p, H, st)
+#define MM_XTI(N) fs_x_inv_tma<T, N>(p, H, st, gate)
 		MM_FS_SWITCH3(p->px, MM_XTI);
 #undef MM_XTI
 	} else if (p->fast_x) {
-#define MM_XI(N) fs_x_inv<T, N>(p, H, st)
+#define MM_XI(N) fs_x_inv<T, N>(p, H, st, gate)
 		MM_FS_SWITCH3(p->px, MM_XI);
 #undef MM_XI
 	} else

@@ -2373,6 +2373,7 @@ struct BDesc {
 	KTab<T> *kt;
 	DevState *ds;
 	BSlot *slot;
+	const int *conv_err;  // set when a staged pass of the member's own convolution gave up waiting (or NULL)
 	double t_end;  // > 0: stop at this time (clamping the last step); 0: stop on the torque test
 	int n, tiles_x, tiles_y, ntiles;
 };
@@ -2524,7 +2525,7 @@ __global__ void k_controller_grp(const BDesc<T> *__restrict__ d, int count, doub
 	const double h = st->h;
 	const double tq2 = st->max_tq2;
 	st->max_tq2 = 0.0;
-	control_attempt<T>(st, d[i].kt, eps_abs, eps_rel, order, fsal, s, nullptr, nullptr);
+	control_attempt<T>(st, d[i].kt, eps_abs, eps_rel, order, fsal, s, nullptr, d[i].conv_err);
 	BState &b = sl->bs;
 	b.attempts++;
 	sl->need_k0 = 0;
@@ -2825,6 +2826,7 @@ mm_status build_rounds(mm_batch *b, cudaStream_t st)
 		d.kt = (KTab<T> *)s->ktab;
 		d.ds = s->dst;
 		d.slot = sl.dev;
+		d.conv_err = conv_timeout_flag(s);
 		d.t_end = sl.t_end;
 		d.n = (int)s->n;
 		const dim3 tg = stage_grid(s->cfg);
@@ -2836,10 +2838,10 @@ mm_status build_rounds(mm_batch *b, cudaStream_t st)
 		for (int c = 0; (size_t)c * BATCH_CHUNK < 3 * s->n; ++c) c3.push_back(make_int2(i, c));
 		for (int c = 0; (size_t)c * BATCH_CHUNK < s->n; ++c) c1.push_back(make_int2(i, c));
 		// a member has one material (region 1) behind its mask, and its states are zero outside it, so
-		// one Ms scales every cell: no region lookups in the forward x pass
+		// one Ms scales every cell: no region lookups in the grouped forward x pass
 		mem.push_back(ConvGroupMember{s->conv, {s->m, s->ys[0], s->ys[1], s->m_lo},
-		                              {s->hd, sizeof(T) == 4 ? s->ynew_lo : nullptr}, nullptr,
-		                              (const T *)s->ms_tab + 1, &sl.dev->active});
+		                              {s->hd, sizeof(T) == 4 ? s->ynew_lo : nullptr}, s->reg, s->ms_tab,
+		                              &sl.dev->active, (const T *)s->ms_tab + 1});
 	}
 	b->dirty = false;
 	if (b->members.empty()) return MM_OK;
