@@ -50,6 +50,32 @@ mm_status scalar_scratch(ScalarScratch **out)
 	return MM_OK;
 }
 
+mm_status setup_alloc(void **p, size_t bytes, cudaStream_t st)
+{
+	static std::mutex mu;
+	static std::vector<cudaMemPool_t> pools;
+	int dev = 0;
+	MM_CUDA(cudaGetDevice(&dev));
+	cudaMemPool_t pool;
+	{
+		std::lock_guard<std::mutex> lock(mu);
+		if ((int)pools.size() <= dev) pools.resize(dev + 1, nullptr);
+		if (!pools[dev]) {
+			cudaMemPoolProps props{};
+			props.allocType = cudaMemAllocationTypePinned;
+			props.location.type = cudaMemLocationTypeDevice;
+			props.location.id = dev;
+			MM_CUDA(cudaMemPoolCreate(&pools[dev], &props));
+			uint64_t keep = 64u << 20;
+			MM_CUDA(cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep));
+		}
+		pool = pools[dev];
+	}
+	return cuda_status(cudaMallocFromPoolAsync(p, bytes, pool, st), "cudaMallocFromPoolAsync");
+}
+
+void setup_free(void *p, cudaStream_t st) { cudaFreeAsync(p, st); }
+
 mm_status scalar_result(ScalarResult *out)
 {
 	struct Ring {

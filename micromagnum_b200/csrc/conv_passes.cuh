@@ -1572,7 +1572,7 @@ mm_status tensor_spectrum(ConvPlan *p, const double *N, bool octant, cudaStream_
 		}
 	}
 	double *work = nullptr;  // the x spectrum, the x-y spectrum, the twiddles
-	MM_CUDA(cudaMallocAsync(&work, (sizeA + sizeB) * sizeof(double) + tw.size() * sizeof(double2), st));
+	MM_TRY(setup_alloc((void **)&work, (sizeA + sizeB) * sizeof(double) + tw.size() * sizeof(double2), st));
 	double *A = work, *B = work + sizeA;
 	double2 *twd = reinterpret_cast<double2 *>(B + sizeB);
 	mm_status r = cuda_status(cudaMemcpyAsync(twd, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, st),
@@ -1622,7 +1622,7 @@ mm_status tensor_spectrum(ConvPlan *p, const double *N, bool octant, cudaStream_
 		}
 		if (r == MM_OK) r = after_launch("k_spec_axis");
 	}
-	cudaFreeAsync(work, st);
+	setup_free(work, st);
 	if (r == MM_OK) r = cuda_status(cudaStreamSynchronize(st), "cudaStreamSynchronize");
 	return r;
 }

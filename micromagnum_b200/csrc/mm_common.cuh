@@ -220,6 +220,12 @@ struct ScalarResult {
 };
 mm_status scalar_result(ScalarResult *out);
 
+// Stream-ordered scratch of an object's set-up, from a pool of the library's own that keeps at most 64 MiB
+// between uses (the rest goes back to the device): allocated and released on every set-up, the
+// device's default pool was mapped and unmapped each time, which took from one to tens of milliseconds.
+mm_status setup_alloc(void **p, size_t bytes, cudaStream_t st);
+void setup_free(void *p, cudaStream_t st);
+
 // Serialises, across host threads, stream captures of the batch rounds against calls that can
 // synchronise the whole device or allocate (instance set-up and tear-down): a device-wide
 // synchronisation while another thread captures would invalidate that capture.

@@ -2021,21 +2021,21 @@ mm_status create_impl(mm_solver *s, int nmat, const mm_material *mats, const uin
 		double *N = nullptr;
 		const bool octant = !tensor && !c.pbc[0] && !c.pbc[1] && !c.pbc[2];
 		if (octant) {
-			MM_CUDA(cudaMallocAsync(&N, sizeof(double) * 6 * s->n, st));
+			MM_TRY(setup_alloc((void **)&N, sizeof(double) * 6 * s->n, st));
 			const mm_status r = tensor_octant(c.nx, c.ny, c.nz, c.dx, c.dy, c.dz, N, st);
-			if (r != MM_OK) { cudaFreeAsync(N, st); return r; }
+			if (r != MM_OK) { setup_free(N, st); return r; }
 		} else if (!tensor) {
-			MM_CUDA(cudaMallocAsync(&N, sizeof(double) * 6 * (size_t)s->px * s->py * s->pz, st));
+			MM_TRY(setup_alloc((void **)&N, sizeof(double) * 6 * (size_t)s->px * s->py * s->pz, st));
 			const int naxes = (c.pbc[0] != 0) + (c.pbc[1] != 0) + (c.pbc[2] != 0);
 			const int repeat = c.pbc_repeat > 0 ? c.pbc_repeat : (naxes == 1 ? 15 : naxes == 2 ? 3 : 2);
 			const mm_status r = mm_demag_tensor_periodic(c.nx, c.ny, c.nz, c.dx, c.dy, c.dz, c.pbc[0] != 0,
 			                                             c.pbc[1] != 0, c.pbc[2] != 0, repeat, s->px, s->py,
 			                                             s->pz, N, st);
-			if (r != MM_OK) { cudaFreeAsync(N, st); return r; }
+			if (r != MM_OK) { setup_free(N, st); return r; }
 		}
 		const mm_status r = conv_plan_create(&s->conv, c.precision, c.nx, c.ny, c.nz, s->px, s->py, s->pz,
 		                                     tensor ? tensor : N, st, keep_lengths, octant);
-		if (N) cudaFreeAsync(N, st);
+		if (N) setup_free(N, st);
 		MM_TRY(r);
 	}
 	MM_TRY((stage_resident<T, sizeof(T) == 4>(&s->st_resident)));
