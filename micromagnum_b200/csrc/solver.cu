@@ -28,7 +28,6 @@
 #include "tma.cuh"
 
 #include <vector>
-#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
@@ -48,19 +47,23 @@ struct DevMat {
 	T j[3];
 };
 
-struct DevState {
-	double t;         // time at the start of the attempt
-	double h;         // step size of the attempt
-	double t_max;     // an accepted attempt that ends past this time is not applied ...
-	int force;        // ... and this one is, whatever its error (both set by the host with t and h)
-	int applied;      // controller output: the accept kernel behind it takes the new state
+// What the host sets for an attempt.
+struct AttemptIn {
+	double t;      // time at the start of the attempt
+	double h;      // step size of the attempt
+	double t_max;  // an accepted attempt that ends past this time is not applied ...
+	int force;     // ... and with force != 0 it is, whatever its error
+	int pad;
+};
+
+struct DevState : AttemptIn {
 	double max_err2;  // max |m_err|^2 of the attempt (reduction)
 	double max_k02;   // max |k_0|^2 of the attempt (reduction)
 	double h_new;     // controller output
 	int accept;
+	int applied;      // the accept kernel behind the controller takes the new state
 	int not_finite;
 	int stage_timeout;  // set by a staged stage kernel whose bounded wait gave up
-	int pad;
 	double max_tq2;   // max (|m x H_eff| / Ms)^2 at the last stage's input (batched relaxations)
 };
 
@@ -1304,6 +1307,7 @@ struct mm_solver {
 	void *ktab = nullptr;                      // KTab<T> on device
 	DevState *dst = nullptr;                   // device state
 	DevState *hst = nullptr;                   // pinned host copy of the controller output
+	AttemptIn *hin = nullptr;                  // pinned inputs of the next attempt; the device only reads them
 	double *avg = nullptr;                     // device scratch for <M>
 	double *avg_h = nullptr;                   // pinned
 	int last_stage_buf = 0;                    // ys[] index holding y_{n+1}
@@ -1438,6 +1442,8 @@ mm_status alloc_state(mm_solver *s)
 	MM_CUDA(cudaMemset(s->dst, 0, sizeof(DevState)));
 	MM_CUDA(cudaMallocHost(&s->hst, sizeof(DevState)));
 	std::memset(s->hst, 0, sizeof(DevState));
+	MM_CUDA(cudaMallocHost(&s->hin, sizeof(AttemptIn)));
+	std::memset(s->hin, 0, sizeof(AttemptIn));
 	MM_CUDA(cudaMalloc(&s->avg, 8 * sizeof(double)));
 	MM_CUDA(cudaMallocHost(&s->avg_h, 8 * sizeof(double)));
 	return MM_OK;
@@ -1787,8 +1793,16 @@ mm_status attempt(mm_solver *s, bool eval_k0, cudaStream_t st)
 	return MM_OK;
 }
 
-// The leading fields of the device state that the host sets per attempt.
-constexpr size_t ATTEMPT_INPUT = offsetof(DevState, applied);
+// The inputs of an attempt that nothing waits for: passed by value, since a pinned copy could be
+// overwritten by the call that follows before the device has read it.
+__global__ void k_put_attempt(DevState *st, AttemptIn in) { *static_cast<AttemptIn *>(st) = in; }
+
+// The pinned inputs in front of an attempt whose end the host waits for (evolve).
+mm_status copy_inputs(mm_solver *s, cudaStream_t st)
+{
+	return cuda_status(cudaMemcpyAsync(static_cast<AttemptIn *>(s->dst), s->hin, sizeof(AttemptIn), cudaMemcpyHostToDevice, st),
+	                   "cudaMemcpyAsync");
+}
 
 template <typename T>
 mm_status controller(mm_solver *s, cudaStream_t st)
@@ -1810,17 +1824,8 @@ mm_status accept_state(mm_solver *s, cudaStream_t st)
 	return MM_OK;
 }
 
-mm_status put_time(mm_solver *s, double t, double h, cudaStream_t st)
-{
-	// the two leading fields of the device state; pinned staging keeps the copy stream-ordered
-	s->hst->t = t;
-	s->hst->h = h;
-	MM_CUDA(cudaMemcpyAsync(s->dst, s->hst, 2 * sizeof(double), cudaMemcpyHostToDevice, st));
-	return MM_OK;
-}
-
 // One attempt, the controller and the accept step (which applies the new state if the controller says
-// so) as a CUDA graph, behind the H2D copy of the attempt's inputs from the pinned host state, replayed
+// so) as a CUDA graph, behind the H2D copy of the attempt's pinned inputs, replayed
 // with a single launch on the caller's stream: the host waits once per attempt and launches nothing else.
 // (With the accept kernel launched by the host afterwards, and the replay on a private stream ordered
 // by two events, a step of a 128x32 film took 142 us, FP32, against 135.)  Kernel parameters never change
@@ -1836,8 +1841,7 @@ mm_status attempt_graph(mm_solver *s, bool eval_k0, cudaStream_t st)
 		st = s->gs;
 		const uint64_t before = launch_counter().load();
 		MM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-		mm_status r = cuda_status(cudaMemcpyAsync(s->dst, s->hst, ATTEMPT_INPUT, cudaMemcpyHostToDevice, st),
-		                          "cudaMemcpyAsync");
+		mm_status r = copy_inputs(s, st);
 		if (r == MM_OK) r = attempt<T>(s, eval_k0, st);
 		if (r == MM_OK) r = controller<T>(s, st);
 		if (r == MM_OK) r = accept_state<T>(s, st);
@@ -1868,13 +1872,10 @@ template <typename T>
 mm_status attempt_and_control(mm_solver *s, double h, double t_max, bool force, cudaStream_t st)
 {
 	const bool eval_k0 = !(s->tab.fsal && s->k0_valid);
-	s->hst->t = s->t;
-	s->hst->h = h;
-	s->hst->t_max = t_max;
-	s->hst->force = force;
+	*s->hin = AttemptIn{s->t, h, t_max, force, 0};
 	if (profiling_on()) {
 		// per-kernel event timing needs direct launches
-		MM_CUDA(cudaMemcpyAsync(s->dst, s->hst, ATTEMPT_INPUT, cudaMemcpyHostToDevice, st));
+		MM_TRY(copy_inputs(s, st));
 		MM_TRY(attempt<T>(s, eval_k0, st));
 		MM_TRY(controller<T>(s, st));
 		MM_TRY(accept_state<T>(s, st));
@@ -1911,12 +1912,15 @@ mm_status evolve(mm_solver *s, double t_max, cudaStream_t st)
 		}
 		break;
 	}
-	if (!s->hst->applied) {  // it ends past t_max
+	const bool past = s->t + h_try > t_max;
+	if (past == (s->hst->applied != 0)) return fail(MM_ERR_CUDA, "solver: the device's accept decision is not the host's");
+	if (past) {
 		// runge_kutta.py:75-78: redo the step with the clamped size, accepted without a check
 		h_try = t_max - s->t;
 		// the controller's decision is ignored; it keeps the reductions reset and the
 		// first-same-as-last swap in step
 		MM_TRY(attempt_and_control<T>(s, h_try, t_max, true, st));
+		if (!s->hst->applied) return fail(MM_ERR_CUDA, "solver: the shortened step was not applied");
 	}
 	s->t += h_try;
 	s->h = h_try;
@@ -1996,6 +2000,7 @@ void free_solver(mm_solver *s)
 	cudaFree(s->ktab);
 	cudaFree(s->dst);
 	cudaFreeHost(s->hst);
+	cudaFreeHost(s->hin);
 	cudaFree(s->avg);
 	cudaFreeHost(s->avg_h);
 	delete s;
@@ -2229,7 +2234,8 @@ MM_API mm_status mm_solver_attempt(mm_solver *s, double h, void *stream)
 {
 	if (!s || !(h > 0)) return fail(MM_ERR_INVALID_ARGUMENT, "mm_solver_attempt: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	MM_TRY(put_time(s, s->t, h, st));
+	k_put_attempt<<<1, 1, 0, st>>>(s->dst, AttemptIn{s->t, h, s->t, 0, 0});
+	MM_TRY(after_launch("k_put_attempt"));
 	const bool eval_k0 = !(s->tab.fsal && s->k0_valid);
 	if (s->cfg.precision == MM_F64) {
 		MM_TRY(attempt<double>(s, eval_k0, st));
