@@ -119,8 +119,8 @@ MM_API mm_status mm_scaled_abs_max(int prec, size_t n, const void *M, const void
  * in the reference: it exists for callers that must not allocate once their set-up is done, such
  * as a process whose free device memory is already reserved by a pool (a late cudaMalloc would
  * fail there) or a step loop that must not meet the synchronisation a cudaMalloc/cudaMallocHost
- * can imply; mm_scaled_abs_max allocates a device accumulator and a pinned host word on its
- * first call on each device.  Scratch is a fixed 512 KiB array in the library's static device
+ * can imply; mm_scaled_abs_max allocates device accumulators and pinned host words on its
+ * first call on each device, and again when more than a multiple of 64 such calls are under way at once.  Scratch is a fixed 512 KiB array in the library's static device
  * memory: at most 65536 partial maxima of 4096 cells, so n is limited to 268,435,456 cells and
  * larger n returns MM_ERR_INVALID_ARGUMENT.  Nothing in the scratch has to start at zero.  The
  * first call on each device (with that device current) looks up the array's address; make it

@@ -76,36 +76,46 @@ mm_status setup_alloc(void **p, size_t bytes, cudaStream_t st)
 
 void setup_free(void *p, cudaStream_t st) { cudaFreeAsync(p, st); }
 
-mm_status scalar_result(ScalarResult *out)
+// Free slots per device.  Slots are allocated a block at a time and kept until process exit: as many as
+// calls were ever under way at once, rounded up (a call that failed keeps its slot out of the list).
+namespace {
+constexpr int SCALAR_BLOCK = 64;
+std::mutex g_scalar_mu;
+std::vector<std::vector<ScalarResult>> g_scalar_free;
+} // namespace
+
+mm_status ScalarLease::take()
 {
-	struct Ring {
+	MM_CUDA(cudaGetDevice(&dev_));
+	std::lock_guard<std::mutex> lock(g_scalar_mu);
+	if ((int)g_scalar_free.size() <= dev_) g_scalar_free.resize(dev_ + 1);
+	std::vector<ScalarResult> &list = g_scalar_free[dev_];
+	if (list.empty()) {
 		ScalarSlot *slots = nullptr;
 		double *host = nullptr;
-		unsigned next = 0;
-	};
-	static std::mutex mu;
-	static std::vector<Ring> rings;
-	int dev = 0;
-	MM_CUDA(cudaGetDevice(&dev));
-	std::lock_guard<std::mutex> lock(mu);
-	if ((int)rings.size() <= dev) rings.resize(dev + 1);
-	Ring &r = rings[dev];
-	if (!r.host) {
-		ScalarSlot *slots = nullptr;
-		MM_CUDA(cudaMalloc(&slots, SCALAR_SLOTS * sizeof(ScalarSlot)));
-		MM_CUDA(cudaMemset(slots, 0, SCALAR_SLOTS * sizeof(ScalarSlot)));
-		MM_CUDA(cudaStreamSynchronize(0));  // (zeroed before a kernel of any stream can use them)
-		const mm_status s = cuda_status(cudaMallocHost(&r.host, SCALAR_SLOTS * sizeof(double)), "cudaMallocHost");
+		MM_CUDA(cudaMalloc(&slots, SCALAR_BLOCK * sizeof(ScalarSlot)));
+		mm_status s = cuda_status(cudaMemset(slots, 0, SCALAR_BLOCK * sizeof(ScalarSlot)), "cudaMemset");
+		// (zeroed before a kernel of any stream can use them)
+		if (s == MM_OK) s = cuda_status(cudaStreamSynchronize(0), "cudaStreamSynchronize");
+		if (s == MM_OK) s = cuda_status(cudaMallocHost(&host, SCALAR_BLOCK * sizeof(double)), "cudaMallocHost");
 		if (s != MM_OK) {
 			cudaFree(slots);
-			r.host = nullptr;
 			return s;
 		}
-		r.slots = slots;
+		for (int q = SCALAR_BLOCK - 1; q >= 0; --q) list.push_back(ScalarResult{slots + q, host + q});
 	}
-	out->slot = r.slots + r.next;
-	out->host = r.host + r.next;
-	r.next = (r.next + 1) % SCALAR_SLOTS;
+	r_ = list.back();
+	list.pop_back();
+	return MM_OK;
+}
+
+mm_status ScalarLease::finish(double *value, cudaStream_t st)
+{
+	MM_CUDA(cudaStreamSynchronize(st));
+	*value = *r_.host;
+	std::lock_guard<std::mutex> lock(g_scalar_mu);
+	g_scalar_free[dev_].push_back(r_);
+	r_ = ScalarResult();
 	return MM_OK;
 }
 

@@ -211,14 +211,23 @@ __device__ __forceinline__ void grid_sum_to_host(ScalarSlot *slot, double *host,
 	block_sum_to(&slot->acc, v);
 	if (threadIdx.x == 0) scalar_finish(slot, host);
 }
-// The next slot of the device's ring (a slot comes up again after SCALAR_SLOTS further calls, each of which
-// waits for its result: that many host threads may be in such calls at once).
-constexpr int SCALAR_SLOTS = 256;
 struct ScalarResult {
 	ScalarSlot *slot = nullptr;
 	double *host = nullptr;
 };
-mm_status scalar_result(ScalarResult *out);
+// A slot held by one call, from its launch until its result has been read: no two calls under way share one,
+// however many threads make them.
+class ScalarLease {
+public:
+	mm_status take();
+	// Waits for the kernel on st, reads its result and returns the slot.
+	mm_status finish(double *value, cudaStream_t st);
+	const ScalarResult &arg() const { return r_; }  // (no slot before take())
+
+private:
+	ScalarResult r_;
+	int dev_ = 0;
+};
 
 // Stream-ordered scratch of an object's set-up, from a pool of the library's own that keeps at most 64 MiB
 // between uses (the rest goes back to the device): allocated and released on every set-up, the

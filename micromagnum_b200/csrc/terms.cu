@@ -77,22 +77,23 @@ mm_status run_exchange(int nx, int ny, int nz, double dx, double dy, double dz, 
                        double *energy_host, cudaStream_t st)
 {
 	const size_t n = (size_t)nx * ny * nz;
-	ScalarResult acc;
-	if (energy_host) MM_TRY(scalar_result(&acc));
+	ScalarLease acc;
+	if (energy_host) MM_TRY(acc.take());
 	const double wx = 1.0 / (dx * dx), wy = 1.0 / (dy * dy), wz = 1.0 / (dz * dz);
 	const T *ms = (const T *)Ms, *a = (const T *)A, *m = (const T *)M;
 	T *h = (T *)H;
 	const int g = grid_for(n);
 #define MM_EXCH(X, Y, Z) \
-	if (px == X && py == Y && pz == Z) k_exchange<T, X, Y, Z><<<g, TPB, 0, st>>>(nx, ny, nz, wx, wy, wz, ms, a, m, h, acc);
+	if (px == X && py == Y && pz == Z) k_exchange<T, X, Y, Z><<<g, TPB, 0, st>>>(nx, ny, nz, wx, wy, wz, ms, a, m, h, acc.arg());
 	MM_EXCH(false, false, false) MM_EXCH(false, false, true) MM_EXCH(false, true, false)
 	MM_EXCH(false, true, true) MM_EXCH(true, false, false) MM_EXCH(true, false, true)
 	MM_EXCH(true, true, false) MM_EXCH(true, true, true)
 #undef MM_EXCH
 	MM_TRY(after_launch("k_exchange"));
 	if (energy_host) {
-		MM_CUDA(cudaStreamSynchronize(st));
-		*energy_host = -MU0 / 2.0 * *acc.host * dx * dy * dz;
+		double e = 0.0;
+		MM_TRY(acc.finish(&e, st));
+		*energy_host = -MU0 / 2.0 * e * dx * dy * dz;
 	}
 	return MM_OK;
 }
@@ -310,14 +311,6 @@ __global__ void __launch_bounds__(TPB) k_rk_error_norm2(size_t n3, double eps_ab
 	grid_sum_to_host(out.slot, out.host, acc);
 }
 
-// Waits for a scalar result and reads it.
-mm_status finish_scalar(const ScalarResult &r, double *out, cudaStream_t st)
-{
-	MM_CUDA(cudaStreamSynchronize(st));
-	*out = *r.host;
-	return MM_OK;
-}
-
 bool bad_prec(int prec) { return prec != MM_F64 && prec != MM_F32; }
 
 } // namespace
@@ -348,18 +341,18 @@ MM_API mm_status mm_uniaxial_anisotropy(int prec, size_t n, const void *axis, co
 	if (bad_prec(prec) || n == 0 || !axis || !k || !Ms || !M || !H)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_uniaxial_anisotropy: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	ScalarResult acc;
-	if (energy_host) MM_TRY(scalar_result(&acc));
+	ScalarLease acc;
+	if (energy_host) MM_TRY(acc.take());
 	if (prec == MM_F64)
 		k_uniaxial<double><<<grid_for(n), TPB, 0, st>>>(n, (const double *)axis, (const double *)k,
 		                                                (const double *)Ms, (const double *)M,
-		                                                (double *)H, acc);
+		                                                (double *)H, acc.arg());
 	else
 		k_uniaxial<float><<<grid_for(n), TPB, 0, st>>>(n, (const float *)axis, (const float *)k,
 		                                               (const float *)Ms, (const float *)M,
-		                                               (float *)H, acc);
+		                                               (float *)H, acc.arg());
 	MM_TRY(after_launch("k_uniaxial"));
-	if (energy_host) return finish_scalar(acc, energy_host, st);
+	if (energy_host) return acc.finish(energy_host, st);
 	return MM_OK;
 }
 
@@ -370,18 +363,18 @@ MM_API mm_status mm_cubic_anisotropy(int prec, size_t n, const void *axis1, cons
 	if (bad_prec(prec) || n == 0 || !axis1 || !axis2 || !k || !Ms || !M || !H)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_cubic_anisotropy: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	ScalarResult acc;
-	if (energy_host) MM_TRY(scalar_result(&acc));
+	ScalarLease acc;
+	if (energy_host) MM_TRY(acc.take());
 	if (prec == MM_F64)
 		k_cubic<double><<<grid_for(n), TPB, 0, st>>>(n, (const double *)axis1, (const double *)axis2,
 		                                             (const double *)k, (const double *)Ms,
-		                                             (const double *)M, (double *)H, acc);
+		                                             (const double *)M, (double *)H, acc.arg());
 	else
 		k_cubic<float><<<grid_for(n), TPB, 0, st>>>(n, (const float *)axis1, (const float *)axis2,
 		                                            (const float *)k, (const float *)Ms,
-		                                            (const float *)M, (float *)H, acc);
+		                                            (const float *)M, (float *)H, acc.arg());
 	MM_TRY(after_launch("k_cubic"));
-	if (energy_host) return finish_scalar(acc, energy_host, st);
+	if (energy_host) return acc.finish(energy_host, st);
 	return MM_OK;
 }
 
@@ -429,17 +422,17 @@ MM_API mm_status mm_scaled_abs_max(int prec, size_t n, const void *M, const void
 	if (bad_prec(prec) || n == 0 || !M || !scale || !result_host)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_scaled_abs_max: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	ScalarResult sc;
-	MM_TRY(scalar_result(&sc));
+	ScalarLease sc;
+	MM_TRY(sc.take());
 	if (prec == MM_F64)
 		k_scaled_abs_max<double><<<grid_for(n), TPB, 0, st>>>(n, (const double *)M,
-		                                                      (const double *)scale, sc);
+		                                                      (const double *)scale, sc.arg());
 	else
 		k_scaled_abs_max<float><<<grid_for(n), TPB, 0, st>>>(n, (const float *)M,
-		                                                     (const float *)scale, sc);
+		                                                     (const float *)scale, sc.arg());
 	MM_TRY(after_launch("k_scaled_abs_max"));
 	double r = 0.0;
-	MM_TRY(finish_scalar(sc, &r, st));
+	MM_TRY(sc.finish(&r, st));
 	*result_host = sqrt(r);
 	return MM_OK;
 }
@@ -450,18 +443,18 @@ MM_API mm_status mm_rk_scaled_error_norm(int prec, size_t n, double eps_abs, dou
 	if (bad_prec(prec) || n == 0 || !y || !y_error || !norm_host)
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_rk_scaled_error_norm: invalid argument");
 	cudaStream_t st = as_stream(stream);
-	ScalarResult sc;
-	MM_TRY(scalar_result(&sc));
+	ScalarLease sc;
+	MM_TRY(sc.take());
 	const size_t n3 = 3 * n;
 	if (prec == MM_F64)
 		k_rk_error_norm2<double><<<grid_for(n3), TPB, 0, st>>>(n3, eps_abs, eps_rel, (const double *)y,
-		                                                       (const double *)y_error, sc);
+		                                                       (const double *)y_error, sc.arg());
 	else
 		k_rk_error_norm2<float><<<grid_for(n3), TPB, 0, st>>>(n3, eps_abs, eps_rel, (const float *)y,
-		                                                      (const float *)y_error, sc);
+		                                                      (const float *)y_error, sc.arg());
 	MM_TRY(after_launch("k_rk_error_norm2"));
 	double r = 0.0;
-	MM_TRY(finish_scalar(sc, &r, st));
+	MM_TRY(sc.finish(&r, st));
 	*norm_host = sqrt(r / (double)n3);
 	return MM_OK;
 }
