@@ -59,16 +59,44 @@ __host__ __device__ __forceinline__ const C *tw_of(const C *base, int n, int R)
 {
 	return base + (size_t)n * (R == 8 ? 2 : 1);
 }
+// The pair of T next to (c, s), a point of the unit circle, whose modulus is closest to one: its own
+// rounding would scale every line of both transforms alike, while an error of the angle turns the
+// inverse back by what the forward transform turned (mul_w).  Among the neighbours one step away, the
+// error of the modulus weighs 16 times that of the angle.
+template <typename T>
+cplx<T> unit_near(long double c, long double s)
+{
+	cplx<T> best{(T)c, (T)s};
+	if (best.x == 0 || best.y == 0) return best;
+	long double least = 1;
+	for (T x : {(T)c, std::nextafter((T)c, T(2)), std::nextafter((T)c, T(-2))})
+		for (T y : {(T)s, std::nextafter((T)s, T(2)), std::nextafter((T)s, T(-2))}) {
+			const long double ex = x - c, ey = y - s, mod = ex * c + ey * s, ang = ey * c - ex * s;
+			const long double cost = 16 * mod * mod + ang * ang;
+			if (cost < least) {
+				least = cost;
+				best = {x, y};
+			}
+		}
+	return best;
+}
+
 template <typename T>
 mm_status make_twiddles(int n, void **out)
 {
 	std::vector<cplx<T>> h((size_t)n * TW_SETS, cplx<T>{0, 0});
-	for (int k = 0; k < n; ++k) {
+	const bool ct = fft_is_pow2(n) || (n % 3 == 0 && fft_is_pow2(n / 3)), oct = ct && n % 8 == 0;
+	// (for the lengths with passes of their own an eighth of the circle, and the rest by symmetry)
+	for (int k = 0; k < (oct ? n / 8 + 1 : n); ++k) {
 		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
-		h[k].x = (T)cosl(a);
-		h[k].y = (T)sinl(a);
+		const long double c = cosl(a), s = sinl(a);
+		h[k] = oct ? unit_near<T>(c, s) : cplx<T>{(T)c, (T)s};
 	}
-	if (fft_is_pow2(n) || (n % 3 == 0 && fft_is_pow2(n / 3)))
+	if (oct) {
+		for (int k = n / 8 + 1; k <= n / 4; ++k) h[k] = {-h[n / 4 - k].y, -h[n / 4 - k].x};
+		for (int k = n / 4 + 1; k < n; ++k) h[k] = {h[k - n / 4].y, -h[k - n / 4].x};
+	}
+	if (ct)
 		for (int R : {fft_is_pow2(n) ? 16 : 24, 8}) {
 			if (n < R || (R == 8 && !fft_is_pow2(n))) continue;
 			cplx<T> *t = h.data() + (tw_of<cplx<T>>(nullptr, n, R) - (const cplx<T> *)nullptr);

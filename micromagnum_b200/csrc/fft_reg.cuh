@@ -13,69 +13,44 @@
 
 namespace mm {
 
-// cos(2 pi q / 64) and cos(2 pi q / 48) for the first quarter, and the rest by symmetry.  Called with
-// constants after unrolling, so the values are operands in the instruction stream: from __constant__
-// tables they were fetched anew by every SM in every launch, which the short launches waited for.
-__host__ __device__ constexpr double cos_q64(int q)
+// cos(2 pi r / n) - 1 and sin(2 pi r / n) for n = 64 or 48, 0 < r < n / 8.  Called with constants after
+// unrolling, so the values are operands in the instruction stream: from __constant__ tables they were
+// fetched anew by every SM in every launch, which the short launches waited for.
+__host__ __device__ constexpr double cosm1_of(int r, int n)
 {
-	switch (q) {
-	case 0: return 1.0;
-	case 1: return 0.99518472667219688624;
-	case 2: return 0.98078528040323044913;
-	case 3: return 0.95694033573220886494;
-	case 4: return 0.92387953251128675613;
-	case 5: return 0.88192126434835502971;
-	case 6: return 0.83146961230254523708;
-	case 7: return 0.77301045336273696081;
-	case 8: return 0.70710678118654752440;
-	case 9: return 0.63439328416364549822;
-	case 10: return 0.55557023301960222474;
-	case 11: return 0.47139673682599764856;
-	case 12: return 0.38268343236508977173;
-	case 13: return 0.29028467725446236764;
-	case 14: return 0.19509032201612826785;
-	case 15: return 0.09801714032956060199;
+	switch (n == 64 ? r : 8 + r) {
+	case 1: return -0.004815273327803113755;
+	case 2: return -0.019214719596769550874;
+	case 3: return -0.043059664267791135064;
+	case 4: return -0.076120467488713243872;
+	case 5: return -0.118078735651644970287;
+	case 6: return -0.168530387697454762921;
+	case 7: return -0.226989546637263039189;
+	case 9: return -0.008555138626189588855;
+	case 10: return -0.034074173710931713250;
+	case 11: return -0.076120467488713243872;
+	case 12: return -0.133974596215561353236;
+	case 13: return -0.206646659708764835420;
 	default: return 0.0;
 	}
 }
-__host__ __device__ constexpr double cos_q48(int q)
+__host__ __device__ constexpr double sin_of(int r, int n)
 {
-	switch (q) {
-	case 0: return 1.0;
-	case 1: return 0.99144486137381041114;
-	case 2: return 0.96592582628906828675;
-	case 3: return 0.92387953251128675613;
-	case 4: return 0.86602540378443864676;
-	case 5: return 0.79335334029123516458;
-	case 6: return 0.70710678118654752440;
-	case 7: return 0.60876142900872063942;
-	case 8: return 0.5;
-	case 9: return 0.38268343236508977173;
-	case 10: return 0.25881904510252076235;
-	case 11: return 0.13052619222005159155;
+	switch (n == 64 ? r : 8 + r) {
+	case 1: return 0.098017140329560601994;
+	case 2: return 0.195090322016128267848;
+	case 3: return 0.290284677254462367636;
+	case 4: return 0.382683432365089771728;
+	case 5: return 0.471396736825997648556;
+	case 6: return 0.555570233019602224743;
+	case 7: return 0.634393284163645498215;
+	case 9: return 0.130526192220051591548;
+	case 10: return 0.258819045102520762349;
+	case 11: return 0.382683432365089771728;
+	case 12: return 0.5;
+	case 13: return 0.608761429008720639416;
 	default: return 0.0;
 	}
-}
-// cos(2 pi q / n) for n = 64 or 48, any q >= 0
-__host__ __device__ constexpr double cos_of(int q, int n)
-{
-	q %= n;
-	if (2 * q > n) q = n - q;
-	const bool neg = 4 * q > n;
-	if (neg) q = n / 2 - q;
-	const double c = n == 64 ? cos_q64(q) : cos_q48(q);
-	return neg ? -c : c;
-}
-// W_n^q = exp(-2 pi i q / n): sin(2 pi q / n) = cos(2 pi (q - n / 4) / n)
-template <typename T>
-__device__ __forceinline__ cplx<T> w64(int q)
-{
-	return {(T)cos_of(q, 64), (T)-cos_of(q + 48, 64)};
-}
-template <typename T>
-__device__ __forceinline__ cplx<T> w48(int q)
-{
-	return {(T)cos_of(q, 48), (T)-cos_of(q + 36, 48)};
 }
 
 __host__ __device__ constexpr bool fft_is_pow2(int n) { return (n & (n - 1)) == 0; }
@@ -99,15 +74,46 @@ __device__ __forceinline__ constexpr int dft_pos(int k)
 	return (k % 3) * (N / 3) + brev_c(k / 3, N / 3);
 }
 
-// v W_64^q (conjugated for the inverse), q a compile-time constant after unrolling.
-template <typename T, bool INV>
-__device__ __forceinline__ cplx<T> mul_w64(cplx<T> v, int q)
+// s sqrt(1/2) and s sqrt(3/4), the constants in two parts.
+template <typename T>
+__device__ __forceinline__ T mul_sqrt_half(T s)
 {
-	if (q == 0) return v;
-	if (q == 16) return mul_mi<INV>(v);
-	cplx<T> w = w64<T>(q);
-	if (INV) w = conjc(w);
-	return cmul(v, w);
+	constexpr double c = 0.70710678118654752440;
+	constexpr T hi = (T)c, lo = sizeof(T) == 4 ? (T)(c - (double)hi) : (T)-4.8336466567264565e-17;
+	return fma(s, hi, s * lo);
+}
+template <typename T>
+__device__ __forceinline__ T mul_sin60(T s)
+{
+	constexpr double c = 0.86602540378443864676;
+	constexpr T hi = (T)c, lo = sizeof(T) == 4 ? (T)(c - (double)hi) : (T)5.0175421109034514e-17;
+	return fma(s, hi, s * lo);
+}
+
+// v W_n^q (conjugated for the inverse), n = 64 or 48, q a compile-time constant after unrolling.  The
+// constants are the same in every line and in both directions of a convolution, so a constant whose
+// modulus is off by its rounding scales what it touches twice, coherently: with W rounded to T they were
+// more than half of the FP32 field's error at lengths 2^k and 3 * 2^k.  So W is a number of quarter turns
+// (exact) and a turn of at most n / 8: 1 + (cos - 1) - i sin, whose rounding is relative to the small
+// parts, in four operations like the plain product; an eighth turn multiplies by sqrt(1/2) in two parts.
+// Against direct sums in 80 bits, 128x32 cells, FP32: 1.14e-7, against 1.47e-7 with rounded twiddles
+// and 1.62e-7 in the mixed-radix passes that these took over; 33x30x3: 0.98e-7, 1.34e-7, 1.36e-7; FP64, 128x32:
+// 2.7e-16, 3.0e-16, 3.3e-16.  An evaluation of a 128x32 film takes about 1% longer, a larger box less.
+template <typename T, bool INV, int n>
+__device__ __forceinline__ cplx<T> mul_w(cplx<T> v, int q)
+{
+	const int k = (8 * q / n + 1) / 2, r = q - k * (n / 4);
+	const bool minus = (r > 0) != INV;  // the turn is 1 - i tan
+	if (r == n / 8 || r == -n / 8) {
+		v = minus ? cplx<T>{v.x + v.y, v.y - v.x} : cplx<T>{v.x - v.y, v.y + v.x};
+		v = {mul_sqrt_half(v.x), mul_sqrt_half(v.y)};
+	} else if (r != 0) {
+		const T c = (T)cosm1_of(r < 0 ? -r : r, n), s = (T)(minus ? -sin_of(r < 0 ? -r : r, n) : sin_of(r < 0 ? -r : r, n));
+		v = {fma(v.x, c, fma(-v.y, s, v.x)), fma(v.x, s, fma(v.y, c, v.y))};
+	}
+#pragma unroll
+	for (int i = 0; i < k; ++i) v = mul_mi<INV>(v);
+	return v;
 }
 
 // Decimation-in-frequency stages over v[0..N): a radix-4 stage stands for the radix-2 stages of spans
@@ -128,9 +134,9 @@ __device__ __forceinline__ void dif_stages(cplx<T> (&v)[N])
 				const C s0 = cadd_pk<PK>(x0, x2), d0 = csub_pk<PK>(x0, x2), s1 = cadd_pk<PK>(x1, x3), d1 = csub_pk<PK>(x1, x3);
 				const int q = j * (64 / (4 * Q));  // W_4Q^j = W_64^q
 				v[b + j] = cadd_pk<PK>(s0, s1);
-				v[b + j + Q] = mul_w64<T, INV>(csub_pk<PK>(s0, s1), 2 * q);
-				v[b + j + 2 * Q] = mul_w64<T, INV>(cadd_mi<INV>(d0, d1), q);
-				v[b + j + 3 * Q] = mul_w64<T, INV>(csub_mi<INV>(d0, d1), 3 * q);
+				v[b + j + Q] = mul_w<T, INV, 64>(csub_pk<PK>(s0, s1), 2 * q);
+				v[b + j + 2 * Q] = mul_w<T, INV, 64>(cadd_mi<INV>(d0, d1), q);
+				v[b + j + 3 * Q] = mul_w<T, INV, 64>(csub_mi<INV>(d0, d1), 3 * q);
 			}
 		}
 		if constexpr (Q >= 2) dif_stages<T, N, INV, Q / 2, PK>(v);
@@ -152,24 +158,18 @@ __device__ __forceinline__ void dft_reg3(cplx<T> (&v)[N])
 	using C = cplx<T>;
 	constexpr int M = N / 3;
 	static_assert(3 * M == N && fft_is_pow2(M) && 48 % N == 0, "3 * 2^k points, at most 48");
-	const T s60 = T(0.86602540378443864676372317075293618);  // sin(60 deg)
 	C y[3][M];
 #pragma unroll
 	for (int j = 0; j < M; ++j) {
 		const C a = v[j], b = v[j + M], c = v[j + 2 * M];
 		const C s = cadd_pk<PK>(b, c), d = csub_pk<PK>(b, c);
 		const C t = C{a.x - T(0.5) * s.x, a.y - T(0.5) * s.y};
-		const C r = mul_mi<INV>(C{s60 * d.x, s60 * d.y});
+		const C r = mul_mi<INV>(C{mul_sin60(d.x), mul_sin60(d.y)});
 		y[0][j] = cadd_pk<PK>(a, s);
 		C y1 = cadd(t, r), y2 = csub(t, r);
 		if (j > 0) {
-			C w1 = w48<T>(j * (48 / N)), w2 = w48<T>(2 * j * (48 / N));
-			if (INV) {
-				w1 = conjc(w1);
-				w2 = conjc(w2);
-			}
-			y1 = cmul(y1, w1);
-			y2 = cmul(y2, w2);
+			y1 = mul_w<T, INV, 48>(y1, j * (48 / N));
+			y2 = mul_w<T, INV, 48>(y2, 2 * j * (48 / N));
 		}
 		y[1][j] = y1;
 		y[2][j] = y2;
@@ -206,9 +206,9 @@ __device__ __forceinline__ void dft_reg_halfzero(cplx<T> (&v)[N])
 			const C x0 = v[j], x1 = v[j + Q];
 			const int q = j * (64 / N);
 			v[j] = cadd_pk<PK>(x0, x1);
-			v[j + Q] = mul_w64<T, false>(csub_pk<PK>(x0, x1), 2 * q);
-			v[j + 2 * Q] = mul_w64<T, false>(cadd_mi<false>(x0, x1), q);
-			v[j + 3 * Q] = mul_w64<T, false>(csub_mi<false>(x0, x1), 3 * q);
+			v[j + Q] = mul_w<T, false, 64>(csub_pk<PK>(x0, x1), 2 * q);
+			v[j + 2 * Q] = mul_w<T, false, 64>(cadd_mi<false>(x0, x1), q);
+			v[j + 3 * Q] = mul_w<T, false, 64>(csub_mi<false>(x0, x1), 3 * q);
 		}
 		if constexpr (Q >= 2) dif_stages<T, N, false, Q / 2, PK>(v);
 	} else if constexpr (N == 2) {
