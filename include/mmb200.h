@@ -189,7 +189,9 @@ MM_API mm_status mm_demag_tensor_periodic(int nx, int ny, int nz, double dx, dou
  * math/conv/SymmetricMatrixVectorConvolution_FFT.cpp:31-65, MatrixVectorConvolution_FFT.cpp:
  * 110-375).  N_device is the tensor in the layout of mm_demag_tensor (FP64); the plan keeps its
  * spectrum in working precision `prec` and owns its scratch.  execute() takes M and writes H in
- * `prec`. */
+ * `prec`.  The plan works with the real part of the tensor's transform (of a tensor that is not symmetric
+ * under inversion, the mean of N(r) and N(-r)) at frequencies ky, kz >= 0, and takes the components xx, yy, zz
+ * to be even along each axis, xy, xz, yz odd along their two, as those of a box of cells are. */
 typedef struct mm_conv mm_conv;
 MM_API mm_status mm_conv_create(mm_conv **out, int prec, int nx, int ny, int nz, int ex, int ey,
                                 int ez, const double *N_device, void *stream);

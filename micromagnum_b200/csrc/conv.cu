@@ -21,6 +21,86 @@ FftRadices fft_factor(int n)
 	return f;
 }
 
+// ---- parts of a tensor by parity -------------------------------------------------------------------
+namespace {
+
+// The eight values of component c at (+-i, +-j, +-k), index bits x, y, z: mirrored.
+__device__ __forceinline__ void mirrored(const double *__restrict__ N, int3 e, int c, int i, int j, int k, double (&v)[8])
+{
+	const int x[2] = {i, i ? e.x - i : 0}, y[2] = {j, j ? e.y - j : 0}, z[2] = {k, k ? e.z - k : 0};
+#pragma unroll
+	for (int s = 0; s < 8; ++s) v[s] = N[(((size_t)z[s >> 2] * e.y + y[s >> 1 & 1]) * e.x + x[s & 1]) * 6 + c];
+}
+__device__ __forceinline__ double part(const double (&v)[8], int parity)
+{
+	double sum = 0;
+#pragma unroll
+	for (int s = 0; s < 8; ++s) sum += __popc(parity & s) & 1 ? -v[s] : v[s];
+	return 0.125 * sum;
+}
+
+// One thread per entry of the octant, the components and then x fastest: both directions of every axis are
+// read in whole lines, once.
+__global__ void __launch_bounds__(256) k_tensor_part(const double *__restrict__ N, int3 e, int3 m, int q, double *__restrict__ out)
+{
+	const size_t cnt = (size_t)6 * m.x * m.y * m.z;
+	for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x) {
+		const int c = (int)(t % 6), i = (int)(t / 6 % m.x), j = (int)(t / 6 / m.x % m.y), k = (int)(t / 6 / m.x / m.y);
+		double v[8];
+		mirrored(N, e, c, i, j, k, v);
+		out[t] = part(v, component_parity(c) ^ q);
+	}
+}
+
+// most[0]: the largest entry, most[1]: the largest of parts 3, 5 and 6
+__global__ void __launch_bounds__(256) k_tensor_parity(const double *__restrict__ N, int3 e, int3 m, double *most)
+{
+	const size_t cnt = (size_t)6 * m.x * m.y * m.z;
+	double all = 0, other = 0;
+	for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x) {
+		const int c = (int)(t % 6), i = (int)(t / 6 % m.x), j = (int)(t / 6 / m.x % m.y), k = (int)(t / 6 / m.x / m.y);
+		double v[8];
+		mirrored(N, e, c, i, j, k, v);
+#pragma unroll
+		for (int s = 0; s < 8; ++s) all = fmax(all, fabs(v[s]));
+		for (int q : {3, 5, 6}) other = fmax(other, fabs(part(v, component_parity(c) ^ q)));
+	}
+	block_max_to(most, all);
+	__syncthreads();
+	block_max_to(most + 1, other);
+}
+
+int part_grid(const int (&m)[3])
+{
+	const size_t want = ((size_t)6 * m[0] * m[1] * m[2] + 255) / 256, most = (size_t)num_sms() * 32;
+	return (int)(want < most ? want : most);
+}
+
+} // namespace
+
+mm_status tensor_part(const double *N, const int (&e)[3], const int (&m)[3], int q, double *out, cudaStream_t st)
+{
+	k_tensor_part<<<part_grid(m), 256, 0, st>>>(N, make_int3(e[0], e[1], e[2]), make_int3(m[0], m[1], m[2]), q, out);
+	return after_launch("k_tensor_part");
+}
+
+mm_status tensor_mixed_parity(const double *N, const int (&e)[3], bool *mixed, cudaStream_t st)
+{
+	const int m[3] = {e[0] / 2 + 1, e[1] / 2 + 1, e[2] / 2 + 1};
+	double *most = nullptr, h[2] = {0, 0};
+	MM_TRY(setup_alloc((void **)&most, sizeof(h), st));
+	mm_status r = cuda_status(cudaMemsetAsync(most, 0, sizeof(h), st), "cudaMemsetAsync");
+	if (r == MM_OK) {
+		k_tensor_parity<<<part_grid(m), 256, 0, st>>>(N, make_int3(e[0], e[1], e[2]), make_int3(m[0], m[1], m[2]), most);
+		r = after_launch("k_tensor_parity");
+	}
+	if (r == MM_OK) r = cuda_status(cudaMemcpyAsync(h, most, sizeof(h), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+	setup_free(most, st);
+	if (r == MM_OK) r = cuda_status(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+	// (entries that vanish by symmetry are sums of a few rounded terms)
+	*mixed = h[1] > 8 * 0x1p-53 * h[0];
+	return r;
+}
 
 size_t ConvPlan::spec_bytes() const
 {
@@ -105,6 +185,9 @@ mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int
 	if (nx <= 0 || ny <= 0 || nz <= 0 || ex < nx || ey < ny || ez < nz || !N ||
 	    (octant && (ex < 2 * nx - 1 || ey < 2 * ny - 1 || ez < 2 * nz - 1)))
 		return fail(MM_ERR_INVALID_ARGUMENT, "conv: invalid sizes or null tensor");
+	bool mixed = false;
+	if (!octant) MM_TRY(tensor_mixed_parity(N, {ex, ey, ez}, &mixed, st));
+	keep_lengths = keep_lengths || mixed;  // (its spectrum depends on the length)
 	auto length = [&](int n, int e, bool z) {
 		return keep_lengths ? e : prec == MM_F64 ? conv_fit_length_f64(n, e, z) : conv_fit_length_f32(n, e, z);
 	};
@@ -129,6 +212,7 @@ mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int
 	p->qy = py / 2 + 1;
 	p->qz = pz / 2 + 1;
 	p->is2d = (nz == 1 && pz == 1);
+	p->mixed_parity = mixed;
 	p->rx = fft_factor(px);
 	p->ry = fft_factor(py);
 	p->rz = fft_factor(pz);

@@ -18,6 +18,7 @@ struct ConvPlan {
 	int xbox_n = 1, xbox_w = 0;     // a spectrum row as xbox_n TMA boxes of xbox_w 8-byte elements
 	int qy = 0, qz = 0;             // py/2 + 1, pz/2 + 1 stored tensor frequencies
 	bool is2d = false;              // nz == 1 && pz == 1
+	bool mixed_parity = false;      // the tensor has parts of other parities (tensor_mixed_parity)
 	bool fast_x = false, fast_y = false, fast_z = false;  // compile-time register-FFT passes (2^k, 3 * 2^k)
 	bool reg_z = false;             // z pass with whole columns in registers (nz <= pz/2, pz up to 32)
 	bool tma_y = false;             // y passes fed by TMA-staged tiles (persistent CTAs)
@@ -57,6 +58,17 @@ struct ConvPlan {
 mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey,
                            int ez, const double *N_device, cudaStream_t st, bool keep_lengths = false,
                            bool octant = false);
+
+// The components xx, xy, xz, yy, yz, zz of a demagnetising tensor are even or odd along each axis (bits x, y,
+// z: odd), which the plan's spectrum relies on.  A tensor that is handed in may have parts of other
+// parities; sorted by what they are multiplied with, part q of component c has the parity c's own ^ q.
+//   q with an odd number of bits: not symmetric under inversion; the transform's real part leaves it out
+//   q = 3, 5, 6: the real part contains it
+__host__ __device__ constexpr int component_parity(int c) { return c == 1 ? 3 : c == 2 ? 5 : c == 4 ? 6 : 0; }
+// Whether the tensor (layout e) has parts 3, 5 or 6 beyond the rounding of its largest entry; waits.
+mm_status tensor_mixed_parity(const double *N, const int (&e)[3], bool *mixed, cudaStream_t st);
+// Part q at the offsets [0, m) of each axis, out[m2][m1][m0][6].
+mm_status tensor_part(const double *N, const int (&e)[3], const int (&m)[3], int q, double *out, cudaStream_t st);
 
 // The tensor's octant of offsets >= 0 of a box without periodic axes, [nz][ny][nx][6] (tensor.cu).
 mm_status tensor_octant(int nx, int ny, int nz, double dx, double dy, double dz, double *N, cudaStream_t st);

@@ -367,13 +367,17 @@ struct SpecPass {
 	size_t oc, oo, ok, oi;       // the output's strides
 	int m, inner;                // offsets given along the axis, inner lines per outer index
 	int a[3], b[3], odd[3];      // the pairs of components and their parity along this axis
+	int part;                    // the tensor's part (0, or 3, 5, 6: tensor_mixed_parity)
+	bool add;                    // adds to the output
+	double scale;                // of the outputs; with signs, the components odd along two axes get -scale (i * i)
+	bool signs;
 };
 
 // One CTA: TB lines of one outer index (blockIdx.y) and one pair (blockIdx.z).  KFAST: the axis is the
 // contiguous one, so a warp loads along it; else along the inner lines.
 template <typename OUT, bool KFAST>
 __global__ void __launch_bounds__(NT) k_spec_axis(SpecPass s, OUT *__restrict__ out, FftRadices rad,
-                                                 const double2 *__restrict__ tw_g, int TB, double scale0, double scale1)
+                                                 const double2 *__restrict__ tw_g, int TB)
 {
 	using C = double2;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -402,15 +406,16 @@ __global__ void __launch_bounds__(NT) k_spec_axis(SpecPass s, OUT *__restrict__ 
 	__syncthreads();
 	C *res = KFAST ? fft_lines<double, false>(b0, b1, len, 1, TB, rad, tw) : fft_lines<double, false>(b0, b1, 1, TB, TB, rad, tw);
 	OUT *oa = out + (size_t)s.a[pr] * s.oc + blockIdx.y * s.oo, *ob = out + (size_t)s.b[pr] * s.oc + blockIdx.y * s.oo;
-	const double sa = s.a[pr] == 1 || s.a[pr] == 2 || s.a[pr] == 4 ? scale1 : scale0;
-	const double sb = s.b[pr] == 1 || s.b[pr] == 2 || s.b[pr] == 4 ? scale1 : scale0;
+	const double sa = s.signs && component_parity(s.a[pr]) != s.part ? -s.scale : s.scale;
+	const double sb = s.signs && component_parity(s.b[pr]) != s.part ? -s.scale : s.scale;
 	for (int e = threadIdx.x; e < TB * q; e += blockDim.x) {
 		const int k = KFAST ? e % q : e / TB, b = KFAST ? e / q : e % TB;
 		if (i0 + b >= s.inner) continue;
 		const C z = res[KFAST ? b * len + k : k * TB + b];
 		const size_t at = k * s.ok + (size_t)(i0 + b) * s.oi;
-		oa[at] = (OUT)(sa * (odd ? z.y : z.x));   // odd: z = i A - B
-		ob[at] = (OUT)(sb * (odd ? -z.x : z.y));
+		const double va = sa * (odd ? z.y : z.x), vb = sb * (odd ? -z.x : z.y);  // odd: z = i A - B
+		oa[at] = (OUT)(s.add ? (double)oa[at] + va : va);
+		ob[at] = (OUT)(s.add ? (double)ob[at] + vb : vb);
 	}
 }
 
@@ -1582,30 +1587,20 @@ mm_status fs_setup(ConvPlan *p)
 }
 
 template <typename T>
-mm_status tensor_spectrum(ConvPlan *p, const double *N, bool octant, cudaStream_t st)
+__global__ void __launch_bounds__(NT) k_round(const double *__restrict__ in, T *__restrict__ out, size_t n)
 {
-	const int n3[3] = {p->nx, p->ny, p->nz}, e3[3] = {p->ex, p->ey, p->ez}, p3[3] = {p->px, p->py, p->pz};
+	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = (T)in[i];
+}
+
+// The three passes over one part of the tensor, octant [m2][m1][m0][6] -> out (OUT = T, or double to add up).
+template <typename OUT>
+mm_status spectrum_passes(const ConvPlan *p, const double *octant, int part, const int (&m)[3], double *A, double *B,
+                          const double2 *const (&tw)[3], OUT *out, cudaStream_t st)
+{
+	const int p3[3] = {p->px, p->py, p->pz};
 	const FftRadices rads[3] = {p->rx, p->ry, p->rz};
-	int m[3];  // offsets of an axis that matter: those of the box, or half a period
-	for (int a = 0; a < 3; ++a) m[a] = e3[a] >= 2 * n3[a] - 1 ? n3[a] : e3[a] / 2 + 1;
 	const size_t hx = p->hx, qy = p->qy, qz = p->qz;
-	const size_t sizeA = 6 * hx * m[1] * m[2], sizeB = 6 * hx * qy * m[2];
-	std::vector<double2> tw;
-	size_t tw_at[3];
-	for (int a = 0; a < 3; ++a) {
-		tw_at[a] = tw.size();
-		for (int k = 0; k < p3[a]; ++k) {
-			const long double w = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)p3[a];
-			tw.push_back(double2{(double)cosl(w), (double)sinl(w)});
-		}
-	}
-	double *work = nullptr;  // the x spectrum, the x-y spectrum, the twiddles
-	MM_TRY(setup_alloc((void **)&work, (sizeA + sizeB) * sizeof(double) + tw.size() * sizeof(double2), st));
-	double *A = work, *B = work + sizeA;
-	double2 *twd = reinterpret_cast<double2 *>(B + sizeB);
-	mm_status r = cuda_status(cudaMemcpyAsync(twd, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, st),
-	                          "cudaMemcpyAsync");
-	const size_t lx = (size_t)(octant ? n3[0] : e3[0]), ly = (size_t)(octant ? n3[1] : e3[1]);
+	mm_status r = MM_OK;
 	for (int ax = 0; ax < 3 && r == MM_OK; ++ax) {
 		SpecPass s{};
 		// pairs of equal parity; xy, xz, yz (components 1, 2, 4) are odd along their two axes
@@ -1613,12 +1608,14 @@ mm_status tensor_spectrum(ConvPlan *p, const double *N, bool octant, cudaStream_
 		for (int q = 0; q < 3; ++q) {
 			s.a[q] = pairs[ax][q][0];
 			s.b[q] = pairs[ax][q][1];
-			s.odd[q] = pairs[ax][q][2];
+			s.odd[q] = pairs[ax][q][2] ^ (part >> ax & 1);
 		}
+		s.part = part;
+		s.scale = 1.0;
 		s.m = m[ax];
 		int outer = 1;
 		if (ax == 0) {
-			s.in = N; s.ic = 1; s.ik = 6; s.ii = 6 * lx; s.io = 6 * lx * ly;
+			s.in = octant; s.ic = 1; s.ik = 6; s.ii = 6 * (size_t)m[0]; s.io = 6 * (size_t)m[0] * m[1];
 			s.ok = 1; s.oi = hx; s.oo = hx * m[1]; s.oc = hx * m[1] * m[2];
 			s.inner = m[1];
 			outer = m[2];
@@ -1635,20 +1632,60 @@ mm_status tensor_spectrum(ConvPlan *p, const double *N, bool octant, cudaStream_
 		const int len = p3[ax], TB = pick_tile(len, 1, sizeof(double2), ax == 0 ? 4 : 16);
 		const size_t smem = (size_t)(2 * TB + 1) * len * sizeof(double2);
 		const dim3 grid((s.inner + TB - 1) / TB, outer, 3);
-		const double2 *t = twd + tw_at[ax];
 		if (ax == 0) {
 			r = set_smem<double>((const void *)k_spec_axis<double, true>, smem);
-			if (r == MM_OK) k_spec_axis<double, true><<<grid, NT, smem, st>>>(s, A, rads[ax], t, TB, 1.0, 1.0);
+			if (r == MM_OK) k_spec_axis<double, true><<<grid, NT, smem, st>>>(s, A, rads[ax], tw[ax], TB);
 		} else if (ax == 1) {
 			r = set_smem<double>((const void *)k_spec_axis<double, false>, smem);
-			if (r == MM_OK) k_spec_axis<double, false><<<grid, NT, smem, st>>>(s, B, rads[ax], t, TB, 1.0, 1.0);
+			if (r == MM_OK) k_spec_axis<double, false><<<grid, NT, smem, st>>>(s, B, rads[ax], tw[ax], TB);
 		} else {
-			// the inverse transforms' 1/(px py pz), and i * i = -1 for the components odd along two axes
-			const double scale = 1.0 / ((double)p3[0] * p3[1] * p3[2]);
-			r = set_smem<T>((const void *)k_spec_axis<T, false>, smem);
-			if (r == MM_OK) k_spec_axis<T, false><<<grid, NT, smem, st>>>(s, (T *)p->tensor, rads[ax], t, TB, scale, -scale);
+			s.scale = 1.0 / ((double)p3[0] * p3[1] * p3[2]);  // the inverse transforms'
+			s.signs = true;
+			s.add = part != 0;
+			r = set_smem<double>((const void *)k_spec_axis<OUT, false>, smem);
+			if (r == MM_OK) k_spec_axis<OUT, false><<<grid, NT, smem, st>>>(s, out, rads[ax], tw[ax], TB);
 		}
 		if (r == MM_OK) r = after_launch("k_spec_axis");
+	}
+	return r;
+}
+
+// N: the octant [nz][ny][nx][6] (octant), or a tensor that was handed in, whose part of the components' own
+// parities is taken (of one that has no other: the tensor itself) and, of mixed parity, the others behind it.
+template <typename T>
+mm_status tensor_spectrum(ConvPlan *p, const double *N, bool octant, cudaStream_t st)
+{
+	const int n3[3] = {p->nx, p->ny, p->nz}, e3[3] = {p->ex, p->ey, p->ez}, p3[3] = {p->px, p->py, p->pz};
+	int m[3];  // offsets of an axis that matter: those of the box, or half a period
+	for (int a = 0; a < 3; ++a) m[a] = e3[a] >= 2 * n3[a] - 1 && !p->mixed_parity ? n3[a] : e3[a] / 2 + 1;
+	const size_t hx = p->hx, qy = p->qy, qz = p->qz;
+	const size_t sizeA = 6 * hx * m[1] * m[2], sizeB = 6 * hx * qy * m[2], sizeS = p->mixed_parity ? 6 * hx * qy * qz : 0;
+	std::vector<double2> tw;
+	size_t tw_at[3];
+	for (int a = 0; a < 3; ++a) {
+		tw_at[a] = tw.size();
+		for (int k = 0; k < p3[a]; ++k) {
+			const long double w = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)p3[a];
+			tw.push_back(double2{(double)cosl(w), (double)sinl(w)});
+		}
+	}
+	double *work = nullptr;  // the x spectrum, the x-y spectrum (and before it the part's octant), the sum of parts, the twiddles
+	MM_TRY(setup_alloc((void **)&work, (sizeA + sizeB + sizeS) * sizeof(double) + tw.size() * sizeof(double2), st));
+	double *A = work, *B = work + sizeA, *S = B + sizeB;
+	double2 *twd = reinterpret_cast<double2 *>(S + sizeS);
+	const double2 *const tws[3] = {twd + tw_at[0], twd + tw_at[1], twd + tw_at[2]};
+	mm_status r = cuda_status(cudaMemcpyAsync(twd, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, st),
+	                          "cudaMemcpyAsync");
+	for (int part : {0, 3, 5, 6}) {
+		if (r != MM_OK || (part && !p->mixed_parity)) break;
+		if (!octant) r = tensor_part(N, e3, m, part, B, st);  // (m <= hx, qy along x, y)
+		if (r != MM_OK) break;
+		r = p->mixed_parity ? spectrum_passes<double>(p, B, part, m, A, B, tws, S, st)
+		                    : spectrum_passes<T>(p, octant ? N : B, part, m, A, B, tws, (T *)p->tensor, st);
+	}
+	if (r == MM_OK && p->mixed_parity) {
+		k_round<T><<<num_sms() * 8, NT, 0, st>>>(S, (T *)p->tensor, sizeS);
+		r = after_launch("k_round");
 	}
 	setup_free(work, st);
 	if (r == MM_OK) r = cuda_status(cudaStreamSynchronize(st), "cudaStreamSynchronize");
