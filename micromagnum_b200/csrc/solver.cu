@@ -1440,10 +1440,9 @@ mm_status alloc_state(mm_solver *s)
 	MM_CUDA(cudaMemcpy(s->ktab, &kt, sizeof(kt), cudaMemcpyHostToDevice));
 	MM_CUDA(cudaMalloc(&s->dst, sizeof(DevState)));
 	MM_CUDA(cudaMemset(s->dst, 0, sizeof(DevState)));
-	MM_CUDA(cudaMallocHost(&s->hst, sizeof(DevState)));
-	std::memset(s->hst, 0, sizeof(DevState));
-	MM_CUDA(cudaMallocHost(&s->hin, sizeof(AttemptIn)));
-	std::memset(s->hin, 0, sizeof(AttemptIn));
+	MM_CUDA(cudaMallocHost(&s->hst, sizeof(DevState) + sizeof(AttemptIn)));  // (hin behind hst)
+	std::memset(s->hst, 0, sizeof(DevState) + sizeof(AttemptIn));
+	s->hin = reinterpret_cast<AttemptIn *>(s->hst + 1);
 	MM_CUDA(cudaMalloc(&s->avg, 8 * sizeof(double)));
 	MM_CUDA(cudaMallocHost(&s->avg_h, 8 * sizeof(double)));
 	return MM_OK;
@@ -2000,7 +1999,6 @@ void free_solver(mm_solver *s)
 	cudaFree(s->ktab);
 	cudaFree(s->dst);
 	cudaFreeHost(s->hst);
-	cudaFreeHost(s->hin);
 	cudaFree(s->avg);
 	cudaFreeHost(s->avg_h);
 	delete s;
