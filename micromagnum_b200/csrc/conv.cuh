@@ -98,7 +98,6 @@ struct ConvGroupMember {
 };
 mm_status conv_group_create(ConvGroup **out, const ConvGroupMember *members, int count, cudaStream_t st);
 mm_status conv_group_execute(ConvGroup *g, int input, int gate, cudaStream_t st, int output = 0);
-int conv_group_launches(const ConvGroup *g);
 void conv_group_destroy(ConvGroup *g);
 // Whether a member with these padded lengths takes the grouped fused y+z pass (which keeps a
 // second, kx-major copy of its reduced tensor).

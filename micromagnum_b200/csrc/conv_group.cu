@@ -404,8 +404,11 @@ struct ConvGroup {
 	static constexpr int POOL = 8;
 	cudaStream_t pool[POOL] = {};
 	cudaEvent_t fork = nullptr, join[POOL] = {};
-	// ... and the members of `solo` beside them
+	// ... and the members of `solo` beside them (made by group_create where there are such members: a
+	// group is made for every relaxation of newly set states, and four streams and five events more took a
+	// tenth of the time of a small batch's call)
 	static constexpr int SOLO = 4;
+	int used_solo = 0;
 	cudaStream_t solo_st[SOLO] = {};
 	cudaEvent_t solo_fork = nullptr, solo_join[SOLO] = {};
 	~ConvGroup()
@@ -897,6 +900,15 @@ mm_status group_create(ConvGroup *g, const ConvGroupMember *m, int count, cudaSt
 	auto rank = [](int pass) { return pass == 6 ? 1 : (pass >= 1 ? pass + 1 : pass); };
 	std::stable_sort(g->lists.begin(), g->lists.end(),
 	                 [&](const ConvGroup::List &a, const ConvGroup::List &b) { return rank(a.pass) < rank(b.pass); });
+	// members on their own: one on the caller's stream when it is alone, else beside the grouped passes
+	if (!g->solo.empty() && (!g->lists.empty() || g->solo.size() > 1)) {
+		g->used_solo = std::min<int>((int)g->solo.size(), ConvGroup::SOLO);
+		MM_CUDA(cudaEventCreateWithFlags(&g->solo_fork, cudaEventDisableTiming));
+		for (int q = 0; q < g->used_solo; ++q) {
+			MM_CUDA(cudaStreamCreateWithFlags(&g->solo_st[q], cudaStreamNonBlocking));
+			MM_CUDA(cudaEventCreateWithFlags(&g->solo_join[q], cudaEventDisableTiming));
+		}
+	}
 	for (int i = 0; i < count; ++i) h[i].flags = m[i].flags;
 	MM_CUDA(cudaMemcpyAsync(g->desc, h.data(), sizeof(GDesc<T>) * count, cudaMemcpyHostToDevice, st));
 	MM_CUDA(cudaStreamSynchronize(st));
@@ -915,11 +927,6 @@ mm_status conv_group_create(ConvGroup **out, const ConvGroupMember *members, int
 	for (int q = 0; q < ConvGroup::POOL && rs == MM_OK; ++q) {
 		rs = cuda_status(cudaStreamCreateWithFlags(&g->pool[q], cudaStreamNonBlocking), "cudaStreamCreate");
 		if (rs == MM_OK) rs = cuda_status(cudaEventCreateWithFlags(&g->join[q], cudaEventDisableTiming), "cudaEventCreate");
-	}
-	if (rs == MM_OK) rs = cuda_status(cudaEventCreateWithFlags(&g->solo_fork, cudaEventDisableTiming), "cudaEventCreate");
-	for (int q = 0; q < ConvGroup::SOLO && rs == MM_OK; ++q) {
-		rs = cuda_status(cudaStreamCreateWithFlags(&g->solo_st[q], cudaStreamNonBlocking), "cudaStreamCreate");
-		if (rs == MM_OK) rs = cuda_status(cudaEventCreateWithFlags(&g->solo_join[q], cudaEventDisableTiming), "cudaEventCreate");
 	}
 	if (rs != MM_OK) {
 		delete g;
@@ -944,16 +951,13 @@ mm_status conv_group_execute(ConvGroup *g, int input, int gate, cudaStream_t st,
 	if (output < 0 || output > 1 || (output == 1 && g->one_output))
 		return fail(MM_ERR_INVALID_ARGUMENT, "conv group: bad output selector");
 	auto rank = [](int pass) { return pass == 6 ? 1 : pass; };
-	// members on their own: one on the caller's stream when it is alone, else beside the grouped passes
-	const bool beside = !g->solo.empty() && (!g->lists.empty() || g->solo.size() > 1);
-	const int used_solo = beside ? std::min<int>((int)g->solo.size(), ConvGroup::SOLO) : 0;
-	if (beside) {
+	if (g->used_solo) {
 		MM_CUDA(cudaEventRecord(g->solo_fork, st));
-		for (int q = 0; q < used_solo; ++q) MM_CUDA(cudaStreamWaitEvent(g->solo_st[q], g->solo_fork, 0));
+		for (int q = 0; q < g->used_solo; ++q) MM_CUDA(cudaStreamWaitEvent(g->solo_st[q], g->solo_fork, 0));
 	}
 	for (size_t k = 0; k < g->solo.size(); ++k) {
 		const ConvGroupMember &m = g->solo[k];
-		cudaStream_t sq = beside ? g->solo_st[k % ConvGroup::SOLO] : st;
+		cudaStream_t sq = g->used_solo ? g->solo_st[k % g->used_solo] : st;
 		MM_TRY(g->prec == MM_F64 ? conv_run_f64(m.plan, (const double *)m.M[input], m.reg, (const double *)m.ms_tab,
 		                                        (double *)m.H[output], sq, m.flags, gate)
 		                         : conv_run_f32(m.plan, (const float *)m.M[input], m.reg, (const float *)m.ms_tab,
@@ -985,14 +989,12 @@ mm_status conv_group_execute(ConvGroup *g, int input, int gate, cudaStream_t st,
 		}
 		i = j;
 	}
-	for (int q = 0; q < used_solo; ++q) {
+	for (int q = 0; q < g->used_solo; ++q) {
 		MM_CUDA(cudaEventRecord(g->solo_join[q], g->solo_st[q]));
 		MM_CUDA(cudaStreamWaitEvent(st, g->solo_join[q], 0));
 	}
 	return MM_OK;
 }
-
-int conv_group_launches(const ConvGroup *g) { return g ? (int)g->lists.size() : 0; }
 
 void conv_group_destroy(ConvGroup *g) { delete g; }
 
