@@ -625,11 +625,15 @@ __global__ void __launch_bounds__(LPB * (N / ct_radix(N))) k_x_inv_ct(const cplx
 // components and three tensor entries per value), so the y spectrum never leaves the SM.  Bound by
 // the latency of its passes for films of up to a few ten thousand cells: 128x32 cells, FP64, 8.6 us
 // against 18.7 in the mixed-radix form (5 CTAs of 32 columns), 500x125 cells 14.7 against 27.2
-// (event-timed, about 6 us of it the timing).
+// (event-timed, about 6 us of it the timing).  A CTA has at most 384 threads, which leaves each the 168
+// registers that a radix-16 butterfly and its twiddles need: at 768 threads the FP32 passes spilled over a
+// kilobyte a thread and an evaluation of 1024x1024 cells took 307 us (mixed radix: 278), against 148 with
+// single columns; 640x480 133 (131), 62 with two; 512x512 51 (78), 42; 2000x400 395 (264), 221.  192
+// threads are no better (640x480: 74, 700x700: 99 against 77).
 __host__ __device__ constexpr int y2d_tb(int n, int csize)
 {
 	int tb = 8;
-	while (tb > 1 && (3L * tb * n * csize > 100 * 1024 || 3 * tb * (n / ct_radix(n)) > (csize == 8 ? 768 : 512))) tb >>= 1;
+	while (tb > 1 && (3L * tb * n * csize > 100 * 1024 || 3 * tb * (n / ct_radix(n)) > 384)) tb >>= 1;
 	return tb;
 }
 
