@@ -50,8 +50,8 @@ struct Gate {
 constexpr int NT = 256;                 // threads per CTA for all passes
 constexpr size_t SMEM_TARGET = 100 * 1024;
 
-// Twiddles of a plan's axis: the plain table W_n^k of the mixed-radix passes and, for powers of two
-// (and three times one) behind it the per-pass tables of the register passes (fft_tw_off), the
+// Twiddles of a plan's axis: the plain table W_n^k of the mixed-radix passes, rounded, and, for powers of
+// two (and three times one) behind it the per-pass tables of the register passes (fft_tw_off), the
 // usual radices first, then those of radix 8.
 constexpr int TW_SETS = 3;
 template <class C>
@@ -86,16 +86,19 @@ mm_status make_twiddles(int n, void **out)
 {
 	std::vector<cplx<T>> h((size_t)n * TW_SETS, cplx<T>{0, 0});
 	const bool ct = fft_is_pow2(n) || (n % 3 == 0 && fft_is_pow2(n / 3)), oct = ct && n % 8 == 0;
+	std::vector<cplx<T>> u(oct ? n : 0);  // the values of the pass tables
 	// (for the lengths with passes of their own an eighth of the circle, and the rest by symmetry)
 	for (int k = 0; k < (oct ? n / 8 + 1 : n); ++k) {
 		const long double a = -2.0L * 3.14159265358979323846264338327950288L * (long double)k / (long double)n;
 		const long double c = cosl(a), s = sinl(a);
-		h[k] = oct ? unit_near<T>(c, s) : cplx<T>{(T)c, (T)s};
+		h[k] = {(T)c, (T)s};
+		if (oct) u[k] = unit_near<T>(c, s);
 	}
-	if (oct) {
-		for (int k = n / 8 + 1; k <= n / 4; ++k) h[k] = {-h[n / 4 - k].y, -h[n / 4 - k].x};
-		for (int k = n / 4 + 1; k < n; ++k) h[k] = {h[k - n / 4].y, -h[k - n / 4].x};
-	}
+	if (oct)
+		for (cplx<T> *w : {h.data(), u.data()}) {
+			for (int k = n / 8 + 1; k <= n / 4; ++k) w[k] = {-w[n / 4 - k].y, -w[n / 4 - k].x};
+			for (int k = n / 4 + 1; k < n; ++k) w[k] = {w[k - n / 4].y, -w[k - n / 4].x};
+		}
 	if (ct)
 		for (int R : {fft_is_pow2(n) ? 16 : 24, 8}) {
 			if (n < R || (R == 8 && !fft_is_pow2(n))) continue;
@@ -104,7 +107,7 @@ mm_status make_twiddles(int n, void **out)
 				const int rp = fft_radix(n, R, p);
 				for (int q = 1; q < rp; ++q)
 					for (int jm = 0; jm < ns; ++jm)
-						t[fft_tw_off(n, R, p) + (q - 1) * ns + jm] = h[(size_t)q * jm * (n / (ns * rp))];
+						t[fft_tw_off(n, R, p) + (q - 1) * ns + jm] = (oct ? u : h)[(size_t)q * jm * (n / (ns * rp))];
 				ns *= rp;
 			}
 		}
