@@ -188,10 +188,9 @@ mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int
 	bool mixed = false;
 	if (!octant) MM_TRY(tensor_mixed_parity(N, {ex, ey, ez}, &mixed, st));
 	keep_lengths = keep_lengths || mixed;  // (its spectrum depends on the length)
-	auto length = [&](int n, int e, bool z) {
-		return keep_lengths ? e : prec == MM_F64 ? conv_fit_length_f64(n, e, z) : conv_fit_length_f32(n, e, z);
-	};
-	const int px = length(nx, ex, false), py = length(ny, ey, false), pz = length(nz, ez, true);
+	int len[3] = {ex, ey, ez};
+	if (!keep_lengths) (prec == MM_F64 ? conv_lengths_f64 : conv_lengths_f32)({nx, ny, nz}, {ex, ey, ez}, len);
+	const int px = len[0], py = len[1], pz = len[2];
 	ConvPlan *p = new ConvPlan();
 	p->prec = prec;
 	p->nx = nx; p->ny = ny; p->nz = nz;

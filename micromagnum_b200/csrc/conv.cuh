@@ -109,10 +109,10 @@ FftRadices fft_factor(int n);
 mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
 mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st,
                        const int *flags = nullptr, int gate = 0);
-int conv_fit_length_f64(int n, int e, bool z);
+void conv_lengths_f64(const int (&n)[3], const int (&e)[3], int (&p)[3]);
 mm_status conv_setup_f32(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
 mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const float *ms_tab, float *H, cudaStream_t st,
                        const int *flags = nullptr, int gate = 0);
-int conv_fit_length_f32(int n, int e, bool z);
+void conv_lengths_f32(const int (&n)[3], const int (&e)[3], int (&p)[3]);
 
 } // namespace mm

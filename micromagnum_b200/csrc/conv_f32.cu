@@ -10,6 +10,6 @@ mm_status conv_run_f32(ConvPlan *p, const float *M, const uint8_t *reg, const fl
 	return execute<float>(p, M, reg, ms_tab, H, st, Gate{flags, gate});
 }
 
-int conv_fit_length_f32(int n, int e, bool z) { return fit_length<float>(n, e, z); }
+void conv_lengths_f32(const int (&n)[3], const int (&e)[3], int (&p)[3]) { choose_lengths<float>(n, e, p); }
 
 } // namespace mm

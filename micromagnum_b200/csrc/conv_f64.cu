@@ -10,6 +10,6 @@ mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const d
 	return execute<double>(p, M, reg, ms_tab, H, st, Gate{flags, gate});
 }
 
-int conv_fit_length_f64(int n, int e, bool z) { return fit_length<double>(n, e, z); }
+void conv_lengths_f64(const int (&n)[3], const int (&e)[3], int (&p)[3]) { choose_lengths<double>(n, e, p); }
 
 } // namespace mm
