@@ -178,23 +178,15 @@ ConvPlan::~ConvPlan()
 
 int conv_launches(const ConvPlan *p) { return p->is2d ? 3 : 5; }
 
-mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey, int ez,
-                           const double *N, cudaStream_t st, bool keep_lengths, bool octant)
+// The plan of n cells and a tensor of layout e at FFT lengths `len`.
+static mm_status plan_at(ConvPlan **out, int prec, const int (&n)[3], const int (&e)[3], const int (&len)[3], bool mixed,
+                         const double *N, bool octant, cudaStream_t st)
 {
-	if (prec != MM_F64 && prec != MM_F32) return fail(MM_ERR_INVALID_ARGUMENT, "conv: bad precision");
-	if (nx <= 0 || ny <= 0 || nz <= 0 || ex < nx || ey < ny || ez < nz || !N ||
-	    (octant && (ex < 2 * nx - 1 || ey < 2 * ny - 1 || ez < 2 * nz - 1)))
-		return fail(MM_ERR_INVALID_ARGUMENT, "conv: invalid sizes or null tensor");
-	bool mixed = false;
-	if (!octant) MM_TRY(tensor_mixed_parity(N, {ex, ey, ez}, &mixed, st));
-	keep_lengths = keep_lengths || mixed;  // (its spectrum depends on the length)
-	int len[3] = {ex, ey, ez};
-	if (!keep_lengths) (prec == MM_F64 ? conv_lengths_f64 : conv_lengths_f32)({nx, ny, nz}, {ex, ey, ez}, len);
 	const int px = len[0], py = len[1], pz = len[2];
 	ConvPlan *p = new ConvPlan();
 	p->prec = prec;
-	p->nx = nx; p->ny = ny; p->nz = nz;
-	p->ex = ex; p->ey = ey; p->ez = ez;
+	p->nx = n[0]; p->ny = n[1]; p->nz = n[2];
+	p->ex = e[0]; p->ey = e[1]; p->ez = e[2];
 	p->px = px; p->py = py; p->pz = pz;
 	p->hx = px / 2 + 1;
 	{
@@ -210,7 +202,7 @@ mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int
 	}
 	p->qy = py / 2 + 1;
 	p->qz = pz / 2 + 1;
-	p->is2d = (nz == 1 && pz == 1);
+	p->is2d = (n[2] == 1 && pz == 1);
 	p->mixed_parity = mixed;
 	p->rx = fft_factor(px);
 	p->ry = fft_factor(py);
@@ -226,6 +218,27 @@ mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int
 	}
 	*out = p;
 	return MM_OK;
+}
+
+mm_status conv_plan_create(ConvPlan **out, int prec, int nx, int ny, int nz, int ex, int ey, int ez,
+                           const double *N, cudaStream_t st, bool keep_lengths, bool octant)
+{
+	if (prec != MM_F64 && prec != MM_F32) return fail(MM_ERR_INVALID_ARGUMENT, "conv: bad precision");
+	if (nx <= 0 || ny <= 0 || nz <= 0 || ex < nx || ey < ny || ez < nz || !N ||
+	    (octant && (ex < 2 * nx - 1 || ey < 2 * ny - 1 || ez < 2 * nz - 1)))
+		return fail(MM_ERR_INVALID_ARGUMENT, "conv: invalid sizes or null tensor");
+	const int n[3] = {nx, ny, nz}, e[3] = {ex, ey, ez};
+	bool mixed = false;
+	if (!octant) MM_TRY(tensor_mixed_parity(N, e, &mixed, st));
+	keep_lengths = keep_lengths || mixed;  // (its spectrum depends on the length)
+	int len[3] = {ex, ey, ez};
+	if (!keep_lengths) (prec == MM_F64 ? conv_lengths_f64 : conv_lengths_f32)(n, e, len);
+	const mm_status r = plan_at(out, prec, n, e, len, mixed, N, octant, st);
+	if (r != MM_ERR_OUT_OF_MEMORY || (len[0] == ex && len[1] == ey && len[2] == ez)) return r;
+	// the plan's lengths need up to 2.2 times the spectrum and 3.4 times the tensor of the tensor's own
+	cudaGetLastError();
+	clear_error();
+	return plan_at(out, prec, n, e, e, mixed, N, octant, st);
 }
 
 mm_status conv_execute(ConvPlan *p, const void *M, const uint8_t *regions, const void *ms_table,

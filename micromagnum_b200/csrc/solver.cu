@@ -2092,29 +2092,39 @@ mm_status solver_create(mm_solver **out, const mm_solver_config *config, int num
 		return fail(MM_ERR_INVALID_ARGUMENT, "mm_solver_create: tolerances and h0 must be positive");
 	if ((size_t)c.nx * c.ny * c.nz > (size_t)1 << 31)
 		return fail(MM_ERR_UNSUPPORTED, "mm_solver_create: more than 2^31 cells");
-	mm_solver *s = new mm_solver();
-	s->cfg = c;
-	s->n = (size_t)c.nx * c.ny * c.nz;
-	s->tab = make_tableau(c.tableau);
-	s->px = mm_round_tensor_dimension(c.nx, c.pbc[0] != 0, c.padding);
-	s->py = mm_round_tensor_dimension(c.ny, c.pbc[1] != 0, c.padding);
-	s->pz = mm_round_tensor_dimension(c.nz, c.pbc[2] != 0, c.padding);
-	if (s->pz > 0 && s->pz < min_pz) s->pz = min_pz;
-	if (s->px <= 0 || s->py <= 0 || s->pz <= 0) {
-		delete s;
-		return fail(MM_ERR_INVALID_ARGUMENT, "mm_solver_create: invalid padding");
+	auto create = [&](mm_solver **made, bool keep_lengths) -> mm_status {
+		mm_solver *s = new mm_solver();
+		s->cfg = c;
+		s->n = (size_t)c.nx * c.ny * c.nz;
+		s->tab = make_tableau(c.tableau);
+		s->px = mm_round_tensor_dimension(c.nx, c.pbc[0] != 0, c.padding);
+		s->py = mm_round_tensor_dimension(c.ny, c.pbc[1] != 0, c.padding);
+		s->pz = mm_round_tensor_dimension(c.nz, c.pbc[2] != 0, c.padding);
+		if (s->pz > 0 && s->pz < min_pz) s->pz = min_pz;
+		if (s->px <= 0 || s->py <= 0 || s->pz <= 0) {
+			delete s;
+			return fail(MM_ERR_INVALID_ARGUMENT, "mm_solver_create: invalid padding");
+		}
+		s->h = c.h0;
+		cudaStream_t st = as_stream(stream);
+		const mm_status r = c.precision == MM_F64
+		                        ? create_impl<double>(s, num_materials, materials_host, regions_host, tensor_device, st, keep_lengths)
+		                        : create_impl<float>(s, num_materials, materials_host, regions_host, tensor_device, st, keep_lengths);
+		if (r != MM_OK) {
+			free_solver(s);
+			return r;
+		}
+		*made = s;
+		return MM_OK;
+	};
+	mm_status r = create(out, min_pz > 1);
+	if (r == MM_ERR_OUT_OF_MEMORY && min_pz <= 1) {
+		// (the state behind a convolution at lengths of the plan's choice may fit behind the tensor's own)
+		cudaGetLastError();
+		clear_error();
+		r = create(out, true);
 	}
-	s->h = c.h0;
-	cudaStream_t st = as_stream(stream);
-	const mm_status r = c.precision == MM_F64
-	                        ? create_impl<double>(s, num_materials, materials_host, regions_host, tensor_device, st, min_pz > 1)
-	                        : create_impl<float>(s, num_materials, materials_host, regions_host, tensor_device, st, min_pz > 1);
-	if (r != MM_OK) {
-		free_solver(s);
-		return r;
-	}
-	*out = s;
-	return MM_OK;
+	return r;
 }
 
 } // namespace
