@@ -429,11 +429,21 @@ int pick_tile(int len, int ncomp, size_t elem, int cap)
 	return tb;
 }
 
+// Lets fn take `bytes` of dynamic shared memory.  The attribute belongs to the kernel, not to a plan, and plans of
+// different lengths share kernels, so it is always set to all that the device allows: set to each plan's
+// own need, a later plan with less would have an earlier one's launches refused.
 template <typename T>
 mm_status set_smem(const void *fn, size_t bytes)
 {
-	if (bytes > 48 * 1024)
-		MM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+	if (bytes <= 48 * 1024) return MM_OK;
+	int dev = 0, most = 0;
+	MM_CUDA(cudaGetDevice(&dev));
+	MM_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+	cudaFuncAttributes a{};
+	MM_CUDA(cudaFuncGetAttributes(&a, fn));
+	most -= (int)a.sharedSizeBytes;
+	if (bytes > (size_t)most) return fail(MM_ERR_UNSUPPORTED, "conv: more shared memory than a block can have");
+	MM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 	return MM_OK;
 }
 
