@@ -105,6 +105,10 @@ int conv_group_fused(int prec, int py, int pz, int nz);
 
 FftRadices fft_factor(int n);
 
+// Twiddles of a plan's axis: a plain table and one per set of pass tables.
+constexpr int TW_SETS = 3;
+inline size_t conv_twiddle_entries(int px, int py, int pz) { return (size_t)TW_SETS * (px + py + pz); }
+
 // conv_f64.cu, conv_f32.cu (flags, gate: a batch member's run flags, see ConvGroupMember)
 mm_status conv_setup_f64(ConvPlan *p, const double *N, bool octant, cudaStream_t st);
 mm_status conv_run_f64(ConvPlan *p, const double *M, const uint8_t *reg, const double *ms_tab, double *H, cudaStream_t st,

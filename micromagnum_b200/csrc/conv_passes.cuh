@@ -53,7 +53,6 @@ constexpr size_t SMEM_TARGET = 100 * 1024;
 // Twiddles of a plan's axis: the plain table W_n^k of the mixed-radix passes, rounded, and, for powers of
 // two (and three times one) behind it the per-pass tables of the register passes (fft_tw_off), the
 // usual radices first, then those of radix 8.
-constexpr int TW_SETS = 3;
 template <class C>
 __host__ __device__ __forceinline__ const C *tw_of(const C *base, int n, int R)
 {

@@ -2884,7 +2884,8 @@ mm_status build_rounds(mm_batch *b, cudaStream_t st)
 }
 
 // Device bytes of one instance: resident (state, stage vectors, spectra, tensor spectrum) and the
-// extra transient peak of its set-up (the FP64 tensor and its FFT workspace).
+// extra transient peak of its set-up: the octant of the FP64 tensor, its x and its x-y half spectra and the
+// FP64 twiddles (tensor_spectrum).  The set-up pool keeps up to 64 MiB of that for the next one.
 void instance_bytes(const mm_batch_instance &q, int prec, size_t *resident, size_t *transient)
 {
 	const size_t s = prec == MM_F32 ? 4 : 8, n = (size_t)q.nx * q.ny * q.nz;
@@ -2900,9 +2901,10 @@ void instance_bytes(const mm_batch_instance &q, int prec, size_t *resident, size
 	const size_t lx = w / E;
 	const size_t vecs = (prec == MM_F32 ? 3 : 1) + 2 + 7 + 1;  // m (+lo, ynew_lo), ys[2], k[7], H_demag
 	const size_t tensor = 6 * qz * qy * hx * s;
-	*resident = vecs * 3 * n * s + n + 3 * (size_t)q.nz * py * lx * 2 * s + tensor + (1 << 16);
+	const size_t twiddles = conv_twiddle_entries(px, py, pz) * 2 * s;
+	*resident = vecs * 3 * n * s + n + 3 * (size_t)q.nz * py * lx * 2 * s + tensor + twiddles + (1 << 16);
 	if (conv_group_fused(prec, py, pz, q.nz)) *resident += tensor;  // the fused pass's kx-major copy
-	*transient = 6 * (size_t)px * py * pz * 8 + (size_t)px * py * pz * 16;
+	*transient = 6 * 8 * (n + hx * q.ny * q.nz + hx * qy * q.nz) + 16 * (size_t)(px + py + pz);
 }
 
 template <typename T>
