@@ -771,8 +771,10 @@ mm_status group_tune(const ConvGroup *g, const ConvGroupMember *m, const std::ve
 // A member large enough to fill the device by itself takes the single-instance passes, which are staged
 // through TMA along every axis where its rows allow: its x passes alone have four times as many tiles
 // as there are SMs.  Depends on the member only, so its arithmetic does not depend on the others.  A
-// round of one 1024x1024x4 FP32 member takes 3.36 ms, against 4.08 in the grouped passes; members a
-// quarter of that size fill no more than a wave and stay grouped.
+// round of FP32 members of 512x400x4 cells, a little above that line: one 0.82 ms, against 1.04 in the grouped
+// passes, four 2.91 against 3.50; 512x512x4 0.91 against 1.12, 3.24 against 3.90; 1024x1024x4 3.35 against
+// 4.05; FP64 512x200x4 0.82 against 0.91, four 3.07 against 3.09; 512x512x4 1.64 against 1.94.  (Below the line:
+// not measured on their own.)
 template <typename T>
 bool group_solo(const ConvPlan *p)
 {

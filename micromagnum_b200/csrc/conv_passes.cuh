@@ -596,7 +596,7 @@ __device__ __forceinline__ void x_inv_ct_body(const cplx<T> *__restrict__ S, T *
 	C *sm = reinterpret_cast<C *>(smem_raw);
 	const int tid = threadIdx.x;
 	const int line = tid / TPL, j0 = tid % TPL;
-	const int rows = 3 * ny * nz, nyz = ny * nz;
+	const int rows = 3 * ny * nz;
 	const int ra = 2 * (blk * LPB + line), rb = ra + 1;
 	const bool va = ra < rows, vb = rb < rows;
 	const int qa = va ? ra : 0, qb = vb ? rb : 0;

@@ -29,9 +29,10 @@ template <typename C>
 __device__ __forceinline__ C csub(C a, C b) { return {a.x - b.x, a.y - b.y}; }
 // Single precision: both components in one packed instruction (add/sub/mul/fma.f32x2, rounded like the
 // scalar ones), which leaves issue slots to the address arithmetic and the shared-memory accesses of
-// passes that are bound by issue: the 512x512x16 slab's eight steps take 23.0 ms, against 23.5 with
-// scalar ones, a batch of 40 members 37.2 against 39.4.  Passes with a warp or two per SM wait for
-// latencies instead and keep the scalar form (a 128x32 film: 2.52 ms, against 2.59 packed).
+// passes that are bound by issue: the 512x512x16 slab's eight steps take 23.4 ms, against 23.8 with
+// scalar ones; 800x300x3 and 520x260x9 cells 5% less; a batch of 40 members the same.  The narrow tiles of the
+// x passes and of the fused 2-D pass wait for latencies instead and keep the scalar form (a 128x32
+// film: 2.52 ms, against 2.59 packed); the y and z passes of small 3-D boxes are packed, within 1% of scalar.
 #define MM_F2_BITS(v) (*reinterpret_cast<const unsigned long long *>(&(v)))
 __device__ __forceinline__ float2 f2_from_bits(unsigned long long r) { return *reinterpret_cast<const float2 *>(&r); }
 __device__ __forceinline__ float2 cadd2(float2 a, float2 b)

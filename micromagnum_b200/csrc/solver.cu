@@ -479,7 +479,7 @@ __device__ __forceinline__ bool cell_rhs_delta(const CellArgs<T> &a, const T *__
 {
 	// Every load first, selections afterwards: with a branch around each neighbour the compiler issued
 	// the neighbours' region ids and values one after another, fourteen memory latencies in a row per
-	// cell.  A round of a batch of 40 members (1.7 million cells) took 3.26 ms, against 3.04 this way (with the
+	// cell.  A round of a batch of 40 members (1.7 million cells) took 3.2 ms, against 3.0 this way (with the
 	// forward x pass's single Ms per member).
 	bool has[6];
 	size_t off[6];
