@@ -74,20 +74,27 @@ __device__ __forceinline__ constexpr int dft_pos(int k)
 	return (k % 3) * (N / 3) + brev_c(k / 3, N / 3);
 }
 
-// s sqrt(1/2) and s sqrt(3/4), the constants in two parts.
-template <typename T>
-__device__ __forceinline__ T mul_sqrt_half(T s)
+// v (hi + lo), a constant in two parts; packed (PK) it is as many instructions as a plain constant.
+template <bool PK, typename T>
+__device__ __forceinline__ cplx<T> mul_parts(cplx<T> v, T hi, T lo)
+{
+	using C = cplx<T>;
+	if constexpr (PK) return cfma2(C{hi, hi}, v, cscale2(C{lo, lo}, v));
+	else return {fma(v.x, hi, v.x * lo), fma(v.y, hi, v.y * lo)};
+}
+template <bool PK, typename T>
+__device__ __forceinline__ cplx<T> mul_sqrt_half(cplx<T> v)
 {
 	constexpr double c = 0.70710678118654752440;
 	constexpr T hi = (T)c, lo = sizeof(T) == 4 ? (T)(c - (double)hi) : (T)-4.8336466567264565e-17;
-	return fma(s, hi, s * lo);
+	return mul_parts<PK, T>(v, hi, lo);
 }
-template <typename T>
-__device__ __forceinline__ T mul_sin60(T s)
+template <bool PK, typename T>
+__device__ __forceinline__ cplx<T> mul_sin60(cplx<T> v)
 {
 	constexpr double c = 0.86602540378443864676;
 	constexpr T hi = (T)c, lo = sizeof(T) == 4 ? (T)(c - (double)hi) : (T)5.0175421109034514e-17;
-	return fma(s, hi, s * lo);
+	return mul_parts<PK, T>(v, hi, lo);
 }
 
 // v W_n^q (conjugated for the inverse), n = 64 or 48, q a compile-time constant after unrolling.  The
@@ -99,14 +106,14 @@ __device__ __forceinline__ T mul_sin60(T s)
 // Against direct sums in 80 bits, 128x32 cells, FP32: 1.14e-7, against 1.47e-7 with rounded twiddles
 // and 1.62e-7 in the mixed-radix passes that these took over; 33x30x3: 0.98e-7, 1.34e-7, 1.36e-7; FP64, 128x32:
 // 2.7e-16, 3.0e-16, 3.3e-16.  An evaluation of a 128x32 film takes about 1% longer, a larger box less.
-template <typename T, bool INV, int n>
+template <typename T, bool INV, int n, bool PK>
 __device__ __forceinline__ cplx<T> mul_w(cplx<T> v, int q)
 {
 	const int k = (8 * q / n + 1) / 2, r = q - k * (n / 4);
 	const bool minus = (r > 0) != INV;  // the turn is 1 - i tan
 	if (r == n / 8 || r == -n / 8) {
 		v = minus ? cplx<T>{v.x + v.y, v.y - v.x} : cplx<T>{v.x - v.y, v.y + v.x};
-		v = {mul_sqrt_half(v.x), mul_sqrt_half(v.y)};
+		v = mul_sqrt_half<PK, T>(v);
 	} else if (r != 0) {
 		const T c = (T)cosm1_of(r < 0 ? -r : r, n), s = (T)(minus ? -sin_of(r < 0 ? -r : r, n) : sin_of(r < 0 ? -r : r, n));
 		v = {fma(v.x, c, fma(-v.y, s, v.x)), fma(v.x, s, fma(v.y, c, v.y))};
@@ -134,9 +141,9 @@ __device__ __forceinline__ void dif_stages(cplx<T> (&v)[N])
 				const C s0 = cadd_pk<PK>(x0, x2), d0 = csub_pk<PK>(x0, x2), s1 = cadd_pk<PK>(x1, x3), d1 = csub_pk<PK>(x1, x3);
 				const int q = j * (64 / (4 * Q));  // W_4Q^j = W_64^q
 				v[b + j] = cadd_pk<PK>(s0, s1);
-				v[b + j + Q] = mul_w<T, INV, 64>(csub_pk<PK>(s0, s1), 2 * q);
-				v[b + j + 2 * Q] = mul_w<T, INV, 64>(cadd_mi<INV>(d0, d1), q);
-				v[b + j + 3 * Q] = mul_w<T, INV, 64>(csub_mi<INV>(d0, d1), 3 * q);
+				v[b + j + Q] = mul_w<T, INV, 64, PK>(csub_pk<PK>(s0, s1), 2 * q);
+				v[b + j + 2 * Q] = mul_w<T, INV, 64, PK>(cadd_mi<INV>(d0, d1), q);
+				v[b + j + 3 * Q] = mul_w<T, INV, 64, PK>(csub_mi<INV>(d0, d1), 3 * q);
 			}
 		}
 		if constexpr (Q >= 2) dif_stages<T, N, INV, Q / 2, PK>(v);
@@ -164,12 +171,12 @@ __device__ __forceinline__ void dft_reg3(cplx<T> (&v)[N])
 		const C a = v[j], b = v[j + M], c = v[j + 2 * M];
 		const C s = cadd_pk<PK>(b, c), d = csub_pk<PK>(b, c);
 		const C t = C{a.x - T(0.5) * s.x, a.y - T(0.5) * s.y};
-		const C r = mul_mi<INV>(C{mul_sin60(d.x), mul_sin60(d.y)});
+		const C r = mul_mi<INV>(mul_sin60<PK, T>(d));
 		y[0][j] = cadd_pk<PK>(a, s);
 		C y1 = cadd(t, r), y2 = csub(t, r);
 		if (j > 0) {
-			y1 = mul_w<T, INV, 48>(y1, j * (48 / N));
-			y2 = mul_w<T, INV, 48>(y2, 2 * j * (48 / N));
+			y1 = mul_w<T, INV, 48, PK>(y1, j * (48 / N));
+			y2 = mul_w<T, INV, 48, PK>(y2, 2 * j * (48 / N));
 		}
 		y[1][j] = y1;
 		y[2][j] = y2;
@@ -206,9 +213,9 @@ __device__ __forceinline__ void dft_reg_halfzero(cplx<T> (&v)[N])
 			const C x0 = v[j], x1 = v[j + Q];
 			const int q = j * (64 / N);
 			v[j] = cadd_pk<PK>(x0, x1);
-			v[j + Q] = mul_w<T, false, 64>(csub_pk<PK>(x0, x1), 2 * q);
-			v[j + 2 * Q] = mul_w<T, false, 64>(cadd_mi<false>(x0, x1), q);
-			v[j + 3 * Q] = mul_w<T, false, 64>(csub_mi<false>(x0, x1), 3 * q);
+			v[j + Q] = mul_w<T, false, 64, PK>(csub_pk<PK>(x0, x1), 2 * q);
+			v[j + 2 * Q] = mul_w<T, false, 64, PK>(cadd_mi<false>(x0, x1), q);
+			v[j + 3 * Q] = mul_w<T, false, 64, PK>(csub_mi<false>(x0, x1), 3 * q);
 		}
 		if constexpr (Q >= 2) dif_stages<T, N, false, Q / 2, PK>(v);
 	} else if constexpr (N == 2) {
