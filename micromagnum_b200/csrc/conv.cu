@@ -39,41 +39,46 @@ __device__ __forceinline__ double part(const double (&v)[8], int parity)
 	return 0.125 * sum;
 }
 
-// One thread per entry of the octant, the components and then x fastest: both directions of every axis are
-// read in whole lines, once.
+// A block takes a stretch of one row (j, k) of the octant, a thread an entry, the components and then x fastest:
+// both directions of every axis are read in whole lines, once, and a row costs no division per entry.
 __global__ void __launch_bounds__(256) k_tensor_part(const double *__restrict__ N, int3 e, int3 m, int q, double *__restrict__ out)
 {
-	const size_t cnt = (size_t)6 * m.x * m.y * m.z;
-	for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x) {
-		const int c = (int)(t % 6), i = (int)(t / 6 % m.x), j = (int)(t / 6 / m.x % m.y), k = (int)(t / 6 / m.x / m.y);
-		double v[8];
-		mirrored(N, e, c, i, j, k, v);
-		out[t] = part(v, component_parity(c) ^ q);
-	}
+	const int t = blockIdx.x * 256 + threadIdx.x, c = t % 6, i = t / 6;
+	if (i >= m.x) return;
+	for (int k = blockIdx.z; k < m.z; k += gridDim.z)
+		for (int j = blockIdx.y; j < m.y; j += gridDim.y) {
+			double v[8];
+			mirrored(N, e, c, i, j, k, v);
+			out[((size_t)k * m.y + j) * m.x * 6 + t] = part(v, component_parity(c) ^ q);
+		}
 }
 
 // most[0]: the largest entry, most[1]: the largest of parts 3, 5 and 6
 __global__ void __launch_bounds__(256) k_tensor_parity(const double *__restrict__ N, int3 e, int3 m, double *most)
 {
-	const size_t cnt = (size_t)6 * m.x * m.y * m.z;
+	const int t = blockIdx.x * 256 + threadIdx.x, c = t % 6, i = t / 6;
 	double all = 0, other = 0;
-	for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x) {
-		const int c = (int)(t % 6), i = (int)(t / 6 % m.x), j = (int)(t / 6 / m.x % m.y), k = (int)(t / 6 / m.x / m.y);
-		double v[8];
-		mirrored(N, e, c, i, j, k, v);
+	if (i < m.x)
+		for (int k = blockIdx.z; k < m.z; k += gridDim.z)
+			for (int j = blockIdx.y; j < m.y; j += gridDim.y) {
+				double v[8];
+				mirrored(N, e, c, i, j, k, v);
 #pragma unroll
-		for (int s = 0; s < 8; ++s) all = fmax(all, fabs(v[s]));
-		for (int q : {3, 5, 6}) other = fmax(other, fabs(part(v, component_parity(c) ^ q)));
-	}
+				for (int s = 0; s < 8; ++s) all = fmax(all, fabs(v[s]));
+				for (int q : {3, 5, 6}) other = fmax(other, fabs(part(v, component_parity(c) ^ q)));
+			}
 	block_max_to(most, all);
 	__syncthreads();
 	block_max_to(most + 1, other);
 }
 
-int part_grid(const int (&m)[3])
+// Blocks over the rows: a few rows each where there are many, to keep the maxima's atomic updates few.
+dim3 part_grid(const int (&m)[3])
 {
-	const size_t want = ((size_t)6 * m[0] * m[1] * m[2] + 255) / 256, most = (size_t)num_sms() * 32;
-	return (int)(want < most ? want : most);
+	const int x = (6 * m[0] + 255) / 256, rows = (num_sms() * 32 + x - 1) / x;
+	const int y = m[1] < rows ? m[1] : rows;
+	const int z = (rows + y - 1) / y;
+	return dim3(x, y, m[2] < z ? m[2] : z);
 }
 
 } // namespace
